@@ -381,78 +381,431 @@ int mxm_unmasked(gbk_matrix* out, const CsrView& a, const CsrView& b, cudaStream
 // ---------------------------------------------------------------------------
 // triangle counting
 
-// 1 where A and its CSC differ (A not symmetric) or a diagonal entry exists
-__global__ void k_sym_loop_check(const int32_t* __restrict__ ap, const int32_t* __restrict__ ai,
-                                 const int32_t* __restrict__ tp, const int32_t* __restrict__ ti, int64_t n,
-                                 int64_t nnz, int* __restrict__ bad) {
-    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e <= n && ap[e] != tp[e]) atomicOr(bad, 1);
-    if (e < nnz && ai[e] != ti[e]) atomicOr(bad, 1);
-    if (e < n) {
-        for (int32_t k = ap[e]; k < ap[e + 1]; ++k)
-            if (ai[k] == (int32_t)e) atomicOr(bad, 2);
+// The count needs each undirected edge once, from its (degree, id)-smaller end
+// (u, v): the triangles are the common entries of N+(u) and N+(v).  On an
+// R-MAT graph of 2^17 vertices no N+ list is longer than 315 entries although
+// the largest degree is 15,743, so every list fits a small hash table in
+// shared memory.  The preparation works on tiles of 256 consecutive entries
+// (a warp each), never on rows: with a thread per row the one thread on a hub
+// row took 1.1 - 1.3 ms in each of two kernels where all of the preparation
+// now takes 45 us (same graph).
+constexpr int kTcTile = 256;
+
+enum { kTcAsymmetric = 1, kTcLoop = 2, kTcDuplicate = 4 };
+
+// deg: row lengths; tile_row: the row of each tile's first entry (n - 1 past
+// the last); *bad gets kTcAsymmetric where A's and the CSC's row starts differ.
+__global__ void __launch_bounds__(256) k_tc_degrees(const int32_t* __restrict__ ap, const int32_t* __restrict__ tp,
+                                                    int64_t n, int64_t ntiles, int32_t* __restrict__ deg,
+                                                    int32_t* __restrict__ tile_row, int* __restrict__ bad) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const bool diff = i <= n && ap[i] != tp[i];
+    if (i < n) {
+        const int32_t b = ap[i], d = ap[i + 1] - b;
+        deg[i] = d;
+        const int64_t end = (int64_t)b + d;
+        for (int64_t t = ((int64_t)b + kTcTile - 1) / kTcTile; t * kTcTile < end; ++t) tile_row[t] = (int32_t)i;
+        if (i == n - 1) tile_row[ntiles] = (int32_t)i;
     }
+    if (__any_sync(0xffffffffu, diff) && (threadIdx.x & 31) == 0) atomicOr(bad, kTcAsymmetric);
 }
 
-// keep edge (u, v) when (deg u, u) < (deg v, v): each undirected edge once,
-// from its lower-degree end
-__device__ __forceinline__ bool oriented(const int32_t* ap, int32_t u, int32_t v) {
-    const int32_t du = ap[u + 1] - ap[u], dv = ap[v + 1] - ap[v];
-    return du < dv || (du == dv && u < v);
-}
-
-__global__ void k_orient_counts(const int32_t* __restrict__ ap, const int32_t* __restrict__ ai, int64_t n,
-                                int32_t* __restrict__ cnt) {
-    const int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (u >= n) return;
-    int32_t c = 0;
-    for (int32_t k = ap[u]; k < ap[u + 1]; ++k) c += oriented(ap, (int32_t)u, ai[k]);
-    cnt[u] = c;
-}
-
-__global__ void k_orient_fill(const int32_t* __restrict__ ap, const int32_t* __restrict__ ai, int64_t n,
-                              const int32_t* __restrict__ op, int32_t* __restrict__ oi, int32_t* __restrict__ orow) {
-    const int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (u >= n) return;
-    int32_t w = op[u];
-    for (int32_t k = ap[u]; k < ap[u + 1]; ++k)
-        if (oriented(ap, (int32_t)u, ai[k])) {
-            oi[w] = ai[k];
-            orow[w] = (int32_t)u;
-            ++w;
-        }
-}
-
-// Sum over oriented edges (u, v) of |N+(u) ∩ N+(v)| (rows sorted by id): a
-// warp per edge, lanes walk the shorter list and binary-search the longer.
-__global__ void k_oriented_triangles(const int32_t* __restrict__ op, const int32_t* __restrict__ oi,
-                                     const int32_t* __restrict__ orow, int64_t m,
-                                     unsigned long long* __restrict__ total) {
+// Marks the oriented entries, one bit each (marks) and their number per tile
+// (cnt; cnt[ntiles] = 0), and checks the pattern: *bad collects kTcAsymmetric
+// (A differs from its CSC), kTcLoop (a diagonal entry) and kTcDuplicate (an
+// entry equal to the one before it in its row).  Each lane searches the rows
+// of its eight entries between the rows of the tile's ends, four independent
+// searches at a time over a few neighbouring row starts.
+__global__ void __launch_bounds__(256) k_tc_mark(const int32_t* __restrict__ ap, const int32_t* __restrict__ ai,
+                                                 const int32_t* __restrict__ ti, const int32_t* __restrict__ deg,
+                                                 const int32_t* __restrict__ tile_row, int64_t nnz, int64_t ntiles,
+                                                 uint32_t* __restrict__ marks, int32_t* __restrict__ cnt,
+                                                 int* __restrict__ bad) {
+    constexpr int kSubs = kTcTile / 32, kHalf = kSubs / 2;
     const int lane = threadIdx.x & 31;
-    const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    unsigned long long mine = 0;
-    for (int64_t e = warp; e < m; e += nwarps) {
-        const int32_t u = orow[e], v = oi[e];
-        const int32_t u0 = op[u], u1 = op[u + 1], v0 = op[v], v1 = op[v + 1];
-        const bool us = (u1 - u0) <= (v1 - v0);
-        const int32_t s0 = us ? u0 : v0, s1 = us ? u1 : v1, l0 = us ? v0 : u0, l1 = us ? v1 : u1;
-        for (int32_t p = s0 + lane; p < s1; p += 32) {
-            const int32_t key = oi[p];
-            int32_t lo = l0, hi = l1;
-            while (lo < hi) {
-                const int32_t mid = (lo + hi) >> 1;
-                if (oi[mid] < key)
-                    lo = mid + 1;
-                else
-                    hi = mid;
+    const int64_t t = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (t >= ntiles) return;  // the whole warp leaves together
+    // the last row with ap[row] <= e lies in [first, last]
+    const int32_t first = tile_row[t], last = tile_row[t + 1];
+    int f = 0;
+    int32_t kept = 0, word = 0;
+    for (int h = 0; h < 2; ++h) {
+        const int64_t e0 = t * kTcTile + 32 * kHalf * h + lane;
+        int32_t c[kHalf], dv[kHalf], lo[kHalf], hi[kHalf];
+#pragma unroll
+        for (int i = 0; i < kHalf; ++i) {
+            const int64_t e = e0 + 32 * i;
+            c[i] = e < nnz ? ai[e] : -1;
+            if (e < nnz && ti[e] != c[i]) f |= kTcAsymmetric;
+        }
+#pragma unroll
+        for (int i = 0; i < kHalf; ++i) {
+            dv[i] = c[i] >= 0 ? __ldg(deg + c[i]) : 0;
+            lo[i] = first;
+            hi[i] = last;
+        }
+        for (int32_t span = last - first; span > 0; span >>= 1) {  // the range halves (rounded down) each step
+#pragma unroll
+            for (int i = 0; i < kHalf; ++i)
+                if (lo[i] < hi[i]) {
+                    const int32_t mid = lo[i] + ((hi[i] - lo[i] + 1) >> 1);
+                    if (__ldg(ap + mid) <= e0 + 32 * i)
+                        lo[i] = mid;
+                    else
+                        hi[i] = mid - 1;
+                }
+        }
+#pragma unroll
+        for (int i = 0; i < kHalf; ++i) {
+            const int64_t e = e0 + 32 * i;
+            bool keep = false;
+            int32_t before = __shfl_up_sync(0xffffffffu, c[i], 1);
+            if (lane == 0 && e > 0 && e < nnz) before = ai[e - 1];
+            if (c[i] >= 0) {
+                const int32_t u = lo[i], du = __ldg(deg + u);
+                if (c[i] == u) f |= kTcLoop;
+                if (before == c[i] && e > __ldg(ap + u)) f |= kTcDuplicate;
+                keep = du < dv[i] || (du == dv[i] && u < c[i]);
             }
-            mine += (lo < l1 && oi[lo] == key);
+            const unsigned m = __ballot_sync(0xffffffffu, keep);
+            kept += __popc(m);
+            if (lane == kHalf * h + i) word = (int32_t)m;
         }
     }
+    if (lane < kSubs) marks[t * kSubs + lane] = (uint32_t)word;
+    if (lane == 0) {
+        cnt[t] = kept;
+        if (t == 0) cnt[ntiles] = 0;
+    }
+    f = __reduce_or_sync(0xffffffffu, f);
+    if (lane == 0 && f) atomicOr(bad, f);
+}
+
+// Oriented entries before entry e (e <= nnz).
+__device__ __forceinline__ int32_t tc_rank(const uint32_t* __restrict__ marks, const int32_t* __restrict__ base,
+                                           int64_t nnz, int32_t e) {
+    const int32_t t = e / kTcTile;
+    int32_t r = base[t];
+    if (e < nnz) {
+        const uint32_t* w = marks + (int64_t)t * (kTcTile / 32);
+        const int in = e % kTcTile;
+        for (int i = 0; i < in / 32; ++i) r += __popc(w[i]);
+        r += __popc(w[in / 32] & ((1u << (in % 32)) - 1u));
+    } else if (e % kTcTile) {
+        r = base[t + 1];
+    }
+    return r;
+}
+
+// The work items of the count.  An edge {v, w} belongs to its end with the
+// longer oriented list (ties: the larger id), v: N+(v) becomes a set in shared
+// memory and the entries of N+(w) are looked up in it, so the lookups are the
+// sum of min(|N+(v)|, |N+(w)|) over the edges (128 M on R-MAT 2^17; with the
+// edge always at its source 252 M).  An item is a vertex v and a run of at
+// most `run` entries of its row, whose ends w it takes the eligible ones of:
+// hub rows are spread over many items.  Classes by |N+(v)|: up to 32 a warp
+// per item; above that a CTA per item, on a bitmap over all vertices while
+// that fits shared memory, otherwise on hash tables of 4096 and 32768 slots,
+// and by search in the list itself above 8192 entries.
+constexpr int kTcClasses = 4;
+constexpr int kTcWarpRun = 128, kTcCtaRun = 256;
+
+struct TcItems {
+    int2* v[kTcClasses];         // (vertex, first entry)
+    int32_t most[kTcClasses];    // largest |N+(v)| of the class
+    int32_t run[kTcClasses];     // entries per item
+};
+
+// op (row starts of the oriented lists) and the items of each class.
+__global__ void __launch_bounds__(256) k_tc_rows(const int32_t* __restrict__ ap, int64_t n, int64_t nnz,
+                                                 const uint32_t* __restrict__ marks, const int32_t* __restrict__ base,
+                                                 const int* __restrict__ bad, int32_t* __restrict__ op, TcItems items,
+                                                 int32_t* __restrict__ nitem) {
+    if (*bad & (kTcAsymmetric | kTcLoop)) return;
+    const int lane = threadIdx.x & 31;
+    const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    int cls = -1;
+    int32_t ab = 0, ae = 0;
+    if (v < n) {
+        ab = ap[v];
+        ae = ap[v + 1];
+        const int32_t b = tc_rank(marks, base, nnz, ab), e = tc_rank(marks, base, nnz, ae);
+        op[v] = b;
+        if (v == n - 1) op[n] = e;
+        if (e - b >= 2)
+            for (cls = 0; e - b > items.most[cls]; ++cls) {}
+    }
+    for (int c = 0; c < kTcClasses; ++c) {
+        const int32_t run = items.run[c];
+        const int32_t cnt = cls == c ? (int32_t)(((int64_t)ae - ab + run - 1) / run) : 0;
+        int32_t incl = cnt;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += y;
+        }
+        const int32_t all = __shfl_sync(0xffffffffu, incl, 31);
+        if (!all) continue;
+        int32_t at = 0;
+        if (lane == 0) at = atomicAdd(nitem + c, all);
+        at = __shfl_sync(0xffffffffu, at, 0) + incl - cnt;
+        for (int32_t i = 0; i < cnt; ++i) items.v[c][at + i] = make_int2((int32_t)v, ab + i * run);
+    }
+}
+
+// oi: the oriented entries' columns, in entry order (a warp per tile).
+__global__ void __launch_bounds__(256) k_tc_fill(const int32_t* __restrict__ ai, int64_t nnz, int64_t ntiles,
+                                                 const uint32_t* __restrict__ marks, const int32_t* __restrict__ base,
+                                                 const int* __restrict__ bad, int32_t* __restrict__ oi) {
+    if (*bad & (kTcAsymmetric | kTcLoop)) return;  // oi has room for the half that a simple graph keeps
+    const int lane = threadIdx.x & 31;
+    const int64_t t = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (t >= ntiles) return;
+    int32_t at = base[t];
+#pragma unroll
+    for (int sub = 0; sub < kTcTile / 32; ++sub) {
+        const uint32_t m = marks[t * (kTcTile / 32) + sub];
+        if ((m >> lane) & 1u) oi[at + __popc(m & ((1u << lane) - 1u))] = ai[t * kTcTile + 32 * sub + lane];
+        at += __popc(m);
+    }
+}
+
+// The sets N+(v) is looked up in.  Each is built and cleared by `nt` threads,
+// thread t, over the list l[0, d).
+
+// Open addressing over int32 slots (-1 empty), at least four per entry: a
+// lookup that misses ends after 1.4 slots on average.
+struct TcHash {
+    int32_t* tab;
+    uint32_t mask;
+    int shift;
+    __device__ void build(const int32_t* __restrict__ l, int32_t d, int t, int nt) {
+        const int lg = max(6, 32 - __clz(4 * d - 1));
+        mask = (1u << lg) - 1u;
+        shift = 32 - lg;
+        for (int k = t; k <= (int)mask; k += nt) tab[k] = -1;
+        if (nt == 32) __syncwarp();
+        else __syncthreads();
+        for (int32_t j = t; j < d; j += nt)
+            for (uint32_t h = slot(l[j]);; h = (h + 1) & mask) {
+                const int32_t old = atomicCAS(tab + h, -1, l[j]);
+                if (old == -1 || old == l[j]) break;
+            }
+    }
+    __device__ void clear(const int32_t*, int32_t, int, int) {}
+    __device__ __forceinline__ uint32_t slot(int32_t key) const { return ((uint32_t)key * 0x9E3779B1u) >> shift; }
+    __device__ __forceinline__ bool has(int32_t key) const {
+        for (uint32_t h = slot(key);; h = (h + 1) & mask) {
+            const int32_t x = tab[h];
+            if (x == key) return true;
+            if (x < 0) return false;
+        }
+    }
+};
+
+// One bit per vertex (all clear between items).  A lookup is one load whatever
+// the keys, where the hash table's slowest lane sets the pace.  The words of a
+// 32-word group are permuted by the higher bits, so that the hub ids of R-MAT
+// graphs (few bits set) spread over the banks.
+struct TcBits {
+    uint32_t* w;
+    __device__ void build(const int32_t* __restrict__ l, int32_t d, int t, int nt) {
+        for (int32_t j = t; j < d; j += nt) atomicOr(w + word(l[j]), 1u << (l[j] & 31));
+    }
+    __device__ void clear(const int32_t* __restrict__ l, int32_t d, int t, int nt) {
+        for (int32_t j = t; j < d; j += nt) w[word(l[j])] = 0;
+    }
+    __device__ __forceinline__ int32_t word(int32_t key) const { return (key >> 5) ^ ((key >> 10) & 31); }
+    __device__ __forceinline__ bool has(int32_t key) const { return (w[word(key)] >> (key & 31)) & 1u; }
+};
+
+// The sorted list itself.
+struct TcSearch {
+    const int32_t* l;
+    int32_t d;
+    __device__ void build(const int32_t* __restrict__ list, int32_t len, int, int) {
+        l = list;
+        d = len;
+    }
+    __device__ void clear(const int32_t*, int32_t, int, int) {}
+    __device__ __forceinline__ bool has(int32_t key) const {
+        int32_t lo = 0, hi = d;
+        while (lo < hi) {
+            const int32_t mid = (lo + hi) >> 1;
+            if (l[mid] < key)
+                lo = mid + 1;
+            else
+                hi = mid;
+        }
+        return lo < d && l[lo] == key;
+    }
+};
+
+// The eligible ends among 32 row entries (w per lane, -1 none): the entries of
+// their oriented lists found in the set of v (d entries).  Each quarter of the
+// warp walks its own lists, 32 entries (four per lane) at a step, and goes on
+// to its next list by itself, so short lists cost an eighth of a warp each and
+// four loads are in flight per lane (R-MAT 2^17: 237 us for k_tc_cta; with the
+// whole warp on one list and one load at a time 355 us).  `slots`: 32 list
+// ranges of the warp.
+template <class Set>
+__device__ __forceinline__ uint32_t tc_lookup(const Set& set, const int32_t* __restrict__ op,
+                                              const int32_t* __restrict__ oi, int32_t v, int32_t d, int32_t w, int lane,
+                                              int2* slots) {
+    constexpr unsigned kAllLanes = 0xffffffffu;
+    const int32_t wb = w >= 0 ? __ldg(op + w) : 0, we = w >= 0 ? __ldg(op + w + 1) : 0;
+    const int32_t dw = we - wb;
+    const bool mine = dw > 0 && (dw < d || (dw == d && w < v));
+    const unsigned todo = __ballot_sync(kAllLanes, mine);
+    const int nl = __popc(todo);
+    if (mine) slots[__popc(todo & ((1u << lane) - 1u))] = make_int2(wb, we);
+    __syncwarp();
+    uint32_t c = 0;
+    int32_t p = 0, e = 0;  // what is left of the quarter's current list
+    for (int at = lane >> 3;;) {
+        if (p >= e && at < nl) {
+            p = slots[at].x;
+            e = slots[at].y;
+            at += 4;
+        }
+        if (!__any_sync(kAllLanes, p < e)) break;
+        int32_t key[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int32_t q = p + 8 * i + (lane & 7);
+            key[i] = q < e ? __ldg(oi + q) : -1;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (key[i] >= 0) c += set.has(key[i]);
+        p += 32;
+    }
+    __syncwarp();
+    return c;
+}
+
+// The CTA's counts into *total with one atomic.
+template <int THREADS>
+__device__ __forceinline__ void tc_add_total(unsigned long long mine, unsigned long long* total) {
+    __shared__ unsigned long long part[THREADS / 32];
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) mine += __shfl_down_sync(0xffffffffu, mine, off);
-    if (lane == 0 && mine) atomicAdd(total, mine);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = mine;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < THREADS / 32; ++w) mine += part[w];
+        if (mine) atomicAdd(total, mine);
+    }
+}
+
+struct TcArgs {
+    const int32_t* ap;
+    const int32_t* ai;
+    const int32_t* op;
+    const int32_t* oi;
+    const int2* items;
+    const int32_t* nitem;
+    const int* bad;
+    unsigned long long* total;
+    int32_t* next;  // the next item to hand out
+    int32_t run;
+    int32_t words;  // of the bitmap
+};
+
+// A warp per item (|N+(v)| <= 32).
+__global__ void __launch_bounds__(256, 8) k_tc_warp(TcArgs a) {
+    __shared__ int32_t tabs[8][128];
+    __shared__ int2 s_slots[8][32];
+    if (*a.bad) return;
+    int2* slots = s_slots[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
+    TcHash set;
+    set.tab = tabs[threadIdx.x >> 5];
+    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    const int32_t ni = *a.nitem;
+    unsigned long long mine = 0;
+    for (int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < ni; i += nw) {
+        const int2 it = a.items[i];
+        const int32_t b = a.op[it.x], d = a.op[it.x + 1] - b;
+        const int32_t end = it.y + min(a.ap[it.x + 1] - it.y, a.run);
+        set.build(a.oi + b, d, lane, 32);
+        __syncwarp();
+        for (int32_t e = it.y; e < end; e += 32)
+            mine += tc_lookup(set, a.op, a.oi, it.x, d, e + lane < end ? a.ai[e + lane] : -1, lane, slots);
+        __syncwarp();
+    }
+    tc_add_total<256>(mine, a.total);
+}
+
+// A CTA per item, items and the 32-entry groups inside them handed out by
+// counters (with vertices in order the CTAs were idle for 28 % of the time, and
+// with equal shares of an item its warps waited at the barrier).  Bound by the
+// lookups (a list entry from L2, then a random shared-memory word): R-MAT 2^17
+// 237 us, and 30 us for k_tc_warp, where a warp per edge with a binary search
+// per entry of the shorter list took 920 us.
+template <class Set, int THREADS>
+__global__ void __launch_bounds__(THREADS, 2048 / THREADS) k_tc_cta(TcArgs a) {
+    extern __shared__ uint32_t smem[];
+    __shared__ int32_t s_item[2], s_group;
+    __shared__ int2 s_slots[THREADS / 32][32];
+    if (*a.bad) return;
+    int2* slots = s_slots[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
+    Set set;
+    if constexpr (std::is_same<Set, TcHash>::value) set.tab = (int32_t*)smem;
+    if constexpr (std::is_same<Set, TcBits>::value) {
+        set.w = smem;
+        for (int i = threadIdx.x; i < a.words; i += THREADS) smem[i] = 0;
+    }
+    const int32_t ni = *a.nitem;
+    unsigned long long mine = 0;
+    if (threadIdx.x == 0) s_item[0] = atomicAdd(a.next, 1);
+    for (int turn = 0;; turn ^= 1) {
+        __syncthreads();  // the item is known, the set clear
+        const int32_t i = s_item[turn];
+        if (i >= ni) break;
+        const int2 it = a.items[i];
+        const int32_t b = a.op[it.x], d = a.op[it.x + 1] - b;
+        const int32_t end = it.y + min(a.ap[it.x + 1] - it.y, a.run);
+        if (threadIdx.x == 0) {
+            s_item[turn ^ 1] = atomicAdd(a.next, 1);
+            s_group = 0;
+        }
+        set.build(a.oi + b, d, threadIdx.x, THREADS);
+        __syncthreads();
+        for (;;) {
+            int32_t g = 0;
+            if (lane == 0) g = atomicAdd(&s_group, 1);
+            const int32_t e = it.y + 32 * __shfl_sync(0xffffffffu, g, 0);
+            if (e >= end) break;
+            mine += tc_lookup(set, a.op, a.oi, it.x, d, e + lane < end ? a.ai[e + lane] : -1, lane, slots);
+        }
+        __syncthreads();
+        set.clear(a.oi + b, d, threadIdx.x, THREADS);
+    }
+    tc_add_total<THREADS>(mine, a.total);
+}
+
+// Patterns with repeated entries: a repeated entry of an edge's shorter list
+// counts each time it is listed (and the longer list's only once), so which
+// list is walked decides the count, and it is the shorter one for every edge.
+__global__ void __launch_bounds__(256) k_tc_duplicates(const int32_t* __restrict__ op, const int32_t* __restrict__ oi,
+                                                       const int32_t* __restrict__ orow, int64_t m,
+                                                       unsigned long long* __restrict__ total) {
+    const int lane = threadIdx.x & 31;
+    const int64_t gw = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    unsigned long long mine = 0;
+    for (int64_t e = gw; e < m; e += nw) {
+        int32_t u = orow[e], v = oi[e];
+        if (op[u + 1] - op[u] > op[v + 1] - op[v]) {
+            const int32_t x = u;
+            u = v;
+            v = x;
+        }
+        TcSearch longer;
+        longer.build(oi + op[v], op[v + 1] - op[v], 0, 0);
+        for (int32_t p = op[u] + lane; p < op[u + 1]; p += 32) mine += longer.has(oi[p]);
+    }
+    tc_add_total<256>(mine, total);
 }
 
 }  // namespace
@@ -470,33 +823,121 @@ extern "C" int gbk_triangle_count(gbk_matrix A, uint64_t* count, void* stream) {
     const CsrView& a = A->csr;
     const CsrView& t = A->csc;
     const int64_t n = a.nrows, nnz = a.nnz;
+    if (nnz == 0) {
+        *count = 0;
+        return GBK_SUCCESS;
+    }
+    // Everything up to the count is queued before the one read-back: the
+    // kernels after k_tc_mark look at its verdict on the device.
+    const int64_t ntiles = (nnz + kTcTile - 1) / kTcTile;
     Scratch dev(s);
-    int* bad = nullptr;
-    unsigned long long* total = nullptr;
-    if (dev.get(&bad, 4) || dev.get(&total, 8)) return GBK_OUT_OF_MEMORY;
-    GBK_CUDA(cudaMemsetAsync(bad, 0, 4, s));
-    GBK_CUDA(cudaMemsetAsync(total, 0, 8, s));
-    k_sym_loop_check<<<nb(std::max<int64_t>(n + 1, nnz)), 256, 0, s>>>(a.ptr, a.idx, t.ptr, t.idx, n, nnz, bad);
+    uint8_t* mem = nullptr;  // bad, class counts, total, then the arrays
+    size_t tb = 0;
+    cub::DeviceScan::ExclusiveSum(nullptr, tb, (int32_t*)nullptr, (int32_t*)nullptr, ntiles + 1, s);
+    auto up = [](size_t b) { return (b + 255) / 256 * 256; };
+    const size_t b_marks = up(4 * (size_t)ntiles * (kTcTile / 32)), b_cnt = up(4 * (size_t)(ntiles + 1)),
+                 b_op = up(4 * (size_t)(n + 1)), b_oi = up(4 * (size_t)(nnz / 2 + 1));
+    // The bitmap serves up to 2^18 vertices (32 KB, six CTAs on an SM); with
+    // more, too few CTAs fit and the hash tables are as fast or faster (whole
+    // call, R-MAT 2^18: 0.91 ms against 1.22 with hash tables, 2^19: 2.35
+    // against 2.21, 2^20: 12.3 against 5.1).
+    const int64_t words = (n + 1023) / 1024 * 32;
+    const bool bits = words <= 8192;
+    TcItems items;
+    const int32_t most[kTcClasses] = {32, bits ? INT_MAX : 1024, bits ? INT_MAX : 8192, INT_MAX};
+    size_t b_items[kTcClasses], b_all = 0;
+    for (int c = 0; c < kTcClasses; ++c) {
+        items.most[c] = most[c];
+        items.run[c] = c == 0 ? kTcWarpRun : kTcCtaRun;
+        // one item per started run: vertices whose lists are longer than the
+        // class below's share nnz / 2 oriented entries
+        const int64_t least = c == 0 ? 2 : (int64_t)most[c - 1] + 1;
+        b_items[c] = up(8 * (size_t)(std::min<int64_t>(n, nnz / 2 / least + 1) + nnz / items.run[c] + 1));
+        if (c > 0 && most[c - 1] == INT_MAX) b_items[c] = 256;
+        b_all += b_items[c];
+    }
+    if (dev.get(&mem, 256 + b_marks + 2 * b_cnt + b_op + b_all + b_oi + up(tb))) {
+        set_error("gbk_triangle_count: out of device memory");
+        return GBK_OUT_OF_MEMORY;
+    }
+    int* bad = (int*)mem;
+    int32_t* nitem = (int32_t*)(mem + 16);
+    unsigned long long* total = (unsigned long long*)(mem + 64);
+    int32_t* next = (int32_t*)(mem + 128);
+    uint8_t* at = mem + 256;
+    auto take = [&](size_t bytes) {
+        uint8_t* p = at;
+        at += bytes;
+        return p;
+    };
+    uint32_t* marks = (uint32_t*)take(b_marks);
+    int32_t* cnt = (int32_t*)take(b_cnt);
+    int32_t* base = (int32_t*)take(b_cnt);
+    int32_t* op = (int32_t*)take(b_op);
+    for (int c = 0; c < kTcClasses; ++c) items.v[c] = (int2*)take(b_items[c]);
+    int32_t* oi = (int32_t*)take(b_oi);
+    void* tmp = take(up(tb));
+    GBK_CUDA(cudaMemsetAsync(mem, 0, 256, s));
+    const unsigned gt = (unsigned)((ntiles + 7) / 8);
+    int32_t* deg = op;  // until k_tc_rows writes the row starts
+    int32_t* tile_row = base;  // until the scan
+    k_tc_degrees<<<nb(n + 1), 256, 0, s>>>(a.ptr, t.ptr, n, ntiles, deg, tile_row, bad);
     GBK_LAUNCHED();
-    int hbad = 0;
-    GBK_CUDA(cudaMemcpyAsync(&hbad, bad, 4, cudaMemcpyDeviceToHost, s));
+    k_tc_mark<<<gt, 256, 0, s>>>(a.ptr, a.idx, t.idx, deg, tile_row, nnz, ntiles, marks, cnt, bad);
+    GBK_LAUNCHED();
+    GBK_CUDA(cub::DeviceScan::ExclusiveSum(tmp, tb, cnt, base, ntiles + 1, s));
+    count_launch(1);
+    k_tc_rows<<<nb(n), 256, 0, s>>>(a.ptr, n, nnz, marks, base, bad, op, items, nitem);
+    GBK_LAUNCHED();
+    k_tc_fill<<<gt, 256, 0, s>>>(a.idx, nnz, ntiles, marks, base, bad, oi);
+    GBK_LAUNCHED();
+    auto args = [&](int c) {
+        return TcArgs{a.ptr, a.idx, op, oi, items.v[c], nitem + c, bad, total, next + c, items.run[c], (int32_t)words};
+    };
+    auto launch_cta = [&](auto kern, int threads, int per_sm, int smem, int c) -> int {
+        GBK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        kern<<<(unsigned)(num_sms() * per_sm), threads, smem, s>>>(args(c));
+        GBK_LAUNCHED();
+        return GBK_SUCCESS;
+    };
+    // a list of d entries ends at d vertices of at least as many entries, so
+    // nnz >= d (d + 1): small graphs cannot reach the larger classes
+    auto reached = [&](int c) { return nnz > ((int64_t)most[c - 1] + 1) * ((int64_t)most[c - 1] + 1); };
+    int rc2 = GBK_SUCCESS;
+    if (bits) {
+        if (reached(1))
+            rc2 = launch_cta(k_tc_cta<TcBits, 256>, 256, 8, (int)words * 4, 1);
+    } else {
+        if (reached(3)) rc2 = launch_cta(k_tc_cta<TcSearch, 256>, 256, 8, 0, 3);
+        if (!rc2 && reached(2)) rc2 = launch_cta(k_tc_cta<TcHash, 1024>, 1024, 1, 4 * 32768, 2);
+        if (!rc2 && reached(1)) rc2 = launch_cta(k_tc_cta<TcHash, 256>, 256, 8, 4 * 4096, 1);
+    }
+    if (rc2) return rc2;
+    k_tc_warp<<<(unsigned)std::min<int64_t>((n + 7) / 8, (int64_t)num_sms() * 8), 256, 0, s>>>(args(0));
+    GBK_LAUNCHED();
+    struct {
+        int bad;
+        int pad[15];
+        unsigned long long total;
+    } head{};
+    GBK_CUDA(cudaMemcpyAsync(&head, mem, sizeof(head), cudaMemcpyDeviceToHost, s));
     GBK_CUDA(cudaStreamSynchronize(s));
-    if (hbad) {
+    if (head.bad & (kTcAsymmetric | kTcLoop)) {
         // not a simple undirected graph: Burkhardt's sum (sum ((A * A) .* A)) / 6 as it stands
         gbk_matrix C = nullptr;
         rc = gbk_mxm_masked(&C, A, A, A, GBK_PLUS_ONE, GBK_I32, stream);
         if (rc) return rc;
         const CsrView& c = C->csr;
-        void* tmp = nullptr;
-        size_t tb = 0;
+        void* rtmp = nullptr;
+        size_t rtb = 0;
         long long* sum = nullptr;
         rc = dev.get(&sum, 8);
         if (!rc) {
-            cub::DeviceReduce::Sum(nullptr, tb, (const int32_t*)c.val, sum, c.nnz, s);
-            rc = dev.get(&tmp, tb);
+            cub::DeviceReduce::Sum(nullptr, rtb, (const int32_t*)c.val, sum, c.nnz, s);
+            rc = dev.get(&rtmp, rtb);
         }
         long long hs = 0;
-        if (!rc && cub::DeviceReduce::Sum(tmp, tb, (const int32_t*)c.val, sum, c.nnz, s) == cudaSuccess &&
+        if (!rc && cub::DeviceReduce::Sum(rtmp, rtb, (const int32_t*)c.val, sum, c.nnz, s) == cudaSuccess &&
             cudaMemcpyAsync(&hs, sum, 8, cudaMemcpyDeviceToHost, s) == cudaSuccess &&
             cudaStreamSynchronize(s) == cudaSuccess) {
             count_launch(1);
@@ -507,35 +948,23 @@ extern "C" int gbk_triangle_count(gbk_matrix A, uint64_t* count, void* stream) {
         gbk_matrix_destroy(C);
         return rc;
     }
-    // symmetric, no self loops: orient by (degree, id) and count each triangle once
-    int32_t *cnt = nullptr, *op = nullptr, *oi = nullptr, *orow = nullptr;
-    if (dev.get(&cnt, 4 * (n + 1)) || dev.get(&op, 4 * (n + 1))) return GBK_OUT_OF_MEMORY;
-    k_orient_counts<<<nb(n), 256, 0, s>>>(a.ptr, a.idx, n, cnt);
-    GBK_LAUNCHED();
-    GBK_CUDA(cudaMemsetAsync(cnt + n, 0, 4, s));
-    {
-        size_t tb = 0;
-        cub::DeviceScan::ExclusiveSum(nullptr, tb, cnt, op, n + 1, s);
-        void* tmp = nullptr;
-        if (dev.get(&tmp, tb)) return GBK_OUT_OF_MEMORY;
-        GBK_CUDA(cub::DeviceScan::ExclusiveSum(tmp, tb, cnt, op, n + 1, s));
-        count_launch(1);
+    if (head.bad & kTcDuplicate) {
+        int32_t m = 0;
+        int32_t* orow = nullptr;
+        GBK_CUDA(cudaMemcpyAsync(&m, op + n, 4, cudaMemcpyDeviceToHost, s));
+        GBK_CUDA(cudaStreamSynchronize(s));
+        if (dev.get(&orow, 4 * (int64_t)m)) return GBK_OUT_OF_MEMORY;
+        if (m > 0) {
+            k_entry_rows<<<nb(m), 256, 0, s>>>(op, n, m, orow);
+            GBK_LAUNCHED();
+            k_tc_duplicates<<<(unsigned)std::min<int64_t>((m + 7) / 8, (int64_t)num_sms() * 8), 256, 0, s>>>(op, oi, orow,
+                                                                                                      m, total);
+            GBK_LAUNCHED();
+        }
+        GBK_CUDA(cudaMemcpyAsync(&head.total, total, 8, cudaMemcpyDeviceToHost, s));
+        GBK_CUDA(cudaStreamSynchronize(s));
     }
-    int32_t m = 0;
-    GBK_CUDA(cudaMemcpyAsync(&m, op + n, 4, cudaMemcpyDeviceToHost, s));
-    GBK_CUDA(cudaStreamSynchronize(s));
-    if (dev.get(&oi, 4 * (int64_t)m) || dev.get(&orow, 4 * (int64_t)m)) return GBK_OUT_OF_MEMORY;
-    k_orient_fill<<<nb(n), 256, 0, s>>>(a.ptr, a.idx, n, op, oi, orow);
-    GBK_LAUNCHED();
-    if (m > 0) {
-        const int64_t warps = std::min<int64_t>(m, (int64_t)num_sms() * 64);
-        k_oriented_triangles<<<(unsigned)((warps * 32 + 255) / 256), 256, 0, s>>>(op, oi, orow, m, total);
-        GBK_LAUNCHED();
-    }
-    unsigned long long ht = 0;
-    GBK_CUDA(cudaMemcpyAsync(&ht, total, 8, cudaMemcpyDeviceToHost, s));
-    GBK_CUDA(cudaStreamSynchronize(s));
-    *count = (uint64_t)ht;
+    *count = head.total;
     return GBK_SUCCESS;
 }
 

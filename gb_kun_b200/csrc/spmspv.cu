@@ -26,7 +26,6 @@ namespace gbk {
 namespace {
 
 constexpr int kPushThreads = 256;
-constexpr int kPushItems = 4;
 
 __device__ __forceinline__ void atomic_min_val(int32_t* p, int32_t v) { atomicMin(p, v); }
 __device__ __forceinline__ void atomic_min_val(float* p, float v) {
@@ -64,27 +63,6 @@ __device__ __forceinline__ void push_atomic(int probe, T* y, int32_t j, T v) {
         atomic_min_val(y + j, S::add(Lim<T>::max(), v));
 }
 
-// Largest k in [0, nf) with offs[k] <= e (offs ascending, offs[nf] > e),
-// found by the whole warp: each round the 31 lanes probe 31 evenly spaced
-// entries of the open range and a ballot keeps the sub-range, so a frontier
-// of n entries takes about log32(n) rounds of one load each.
-__device__ __forceinline__ int64_t warp_find_entry(const int32_t* __restrict__ offs, int64_t nf, int64_t e,
-                                                   int lane) {
-    int64_t lo = 0, hi = nf;  // offs[lo] <= e < offs[hi] (offs[nf] = E > e)
-    while (hi - lo > 1) {
-        const int64_t span = hi - lo;
-        const int64_t p = lo + (span * (lane + 1) + 31) / 32;  // lanes 0..30 probe inside (lo, hi]
-        const bool le = lane < 31 && p < hi && offs[p] <= e;
-        const unsigned bal = __ballot_sync(0xffffffffu, le);
-        const int c = __popc(bal);  // a prefix of the lanes (offs ascends)
-        const int64_t p_c = __shfl_sync(0xffffffffu, p, c < 31 ? c : 30);
-        const int64_t p_last = __shfl_sync(0xffffffffu, p, c > 0 ? c - 1 : 0);
-        if (c > 0) lo = p_last;
-        if (c < 31) hi = p_c;
-    }
-    return lo;
-}
-
 constexpr int kPushSubTiles = 8;  // 32-edge sub-tiles per warp tile
 
 // One warp per tile of 256 consecutive frontier edges (grid-stride over
@@ -109,39 +87,10 @@ __global__ void __launch_bounds__(kPushThreads) k_push(const int32_t* __restrict
         for (int sub = 0; sub < kPushSubTiles; ++sub) {
             const int64_t e0 = t * kTile + 32 * sub;
             if (e0 >= E) break;
-            const int32_t start0 = offs[k0];
-            // boundary of entry k0 + 1 + lane (E past the last entry)
-            const int64_t kb = k0 + 1 + lane;
-            const int32_t b = kb <= nf ? offs[kb] : (int32_t)E;
             const int64_t e = e0 + lane;
             const bool valid = e < E;
-            // cnt = boundaries <= e among the 32 (they ascend with the lane)
-            int cnt = 0;
-#pragma unroll
-            for (int step = 16; step >= 1; step >>= 1) {
-                const int32_t bv = __shfl_sync(kFull, b, cnt + step - 1);
-                if (bv <= e) cnt += step;
-            }
-            const int32_t b31 = __shfl_sync(kFull, b, 31);
-            const int32_t prev = __shfl_sync(kFull, b, cnt > 0 ? cnt - 1 : 0);
-            int64_t k;
             int32_t start;
-            if (valid && cnt == 31 && b31 <= e) {
-                // more than 32 entries end before this edge (empty rows): search on
-                int64_t lo = k0 + 32, hi = nf;
-                while (hi - lo > 1) {
-                    const int64_t mid = (lo + hi) >> 1;
-                    if (offs[mid] <= e)
-                        lo = mid;
-                    else
-                        hi = mid;
-                }
-                k = lo;
-                start = offs[k];
-            } else {
-                k = k0 + cnt;  // an entry of the frontier for every valid lane
-                start = cnt > 0 ? prev : start0;
-            }
+            const int64_t k = warp_entry_of(offs, nf, k0, e, E, lane, &start);
             int32_t j = -1 - lane;  // a key no other lane has
             T m = S::identity();
             if (valid) {
