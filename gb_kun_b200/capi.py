@@ -215,18 +215,33 @@ def ptr(t) -> C.c_void_p | None:
     return C.c_void_p(t.data_ptr())
 
 
+_DTYPES = None
+
+
 def dtype_code(t) -> int:
-    import torch
-    m = {torch.float32: F32, torch.int32: I32, torch.bool: BOOL, torch.uint8: BOOL, torch.int64: I64,
-         torch.float64: F64}
-    return m[t.dtype]
+    global _DTYPES
+    if _DTYPES is None:
+        import torch
+        _DTYPES = {torch.float32: F32, torch.int32: I32, torch.bool: BOOL, torch.uint8: BOOL, torch.int64: I64,
+                   torch.float64: F64}
+    return _DTYPES[t.dtype]
+
+
+_RAW_STREAM = None
 
 
 def stream_ptr(stream=None):
-    if stream is None:
+    """The cudaStream_t of `stream`, or of torch's current stream on the current device."""
+    global _RAW_STREAM
+    if stream is not None:
+        return C.c_void_p(stream.cuda_stream)
+    if _RAW_STREAM is None:
         import torch
-        stream = torch.cuda.current_stream()
-    return C.c_void_p(stream.cuda_stream)
+        torch.cuda.current_stream()  # initialises CUDA in torch
+        # the handle alone: building torch's Stream object costs more than the rest of a call's arguments
+        device, raw = torch._C._cuda_getDevice, torch._C._cuda_getCurrentRawStream
+        _RAW_STREAM = lambda: raw(device())  # noqa: E731
+    return C.c_void_p(_RAW_STREAM())
 
 
 class Matrix:

@@ -39,6 +39,11 @@ int cuda_fail(cudaError_t e, const char* what, const char* file, int line);
     } while (0)
 
 int num_sms();
+// The calling thread's page of mapped pinned memory (NULL when there is none),
+// and a small device-to-host copy through it that synchronises the stream.
+constexpr size_t kHostPage = 4096;
+void* host_page();
+int read_back(void* dst, const void* src, size_t bytes, cudaStream_t s);
 void count_launch(int n);
 // Loads the allocation-free conversion's module and caches its scratch
 // address for `device` (current); noalloc.cu.

@@ -40,6 +40,40 @@ int num_sms() {
     return g_num_sms;
 }
 
+// One page of mapped pinned memory per host thread for the small results of
+// synchronising calls: a kernel writes it (or a copy fills it) and the thread
+// reads it after its stream, without the staging of a copy to pageable memory.
+// Only that thread's running call uses it.  NULL when none can be had.
+namespace {
+struct HostPage {
+    void* p = nullptr;
+    bool tried = false;
+    ~HostPage() {
+        if (p) cudaFreeHost(p);
+    }
+};
+}  // namespace
+
+void* host_page() {
+    static thread_local HostPage page;
+    if (!page.tried) {
+        page.tried = true;
+        if (cudaHostAlloc(&page.p, kHostPage, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+            page.p = nullptr;
+            cudaGetLastError();
+        }
+    }
+    return page.p;
+}
+
+int read_back(void* dst, const void* src, size_t bytes, cudaStream_t s) {
+    void* page = bytes <= kHostPage ? host_page() : nullptr;
+    GBK_CUDA(cudaMemcpyAsync(page ? page : dst, src, bytes, cudaMemcpyDeviceToHost, s));
+    GBK_CUDA(cudaStreamSynchronize(s));
+    if (page) std::memcpy(dst, page, bytes);
+    return GBK_SUCCESS;
+}
+
 // add(3, 5) in the semiring's element type (src/backend/spmspv/spmspv.h:117).
 int semiring_probe(int sr, int dtype) {
     (void)dtype;

@@ -920,8 +920,8 @@ extern "C" int gbk_triangle_count(gbk_matrix A, uint64_t* count, void* stream) {
         int pad[15];
         unsigned long long total;
     } head{};
-    GBK_CUDA(cudaMemcpyAsync(&head, mem, sizeof(head), cudaMemcpyDeviceToHost, s));
-    GBK_CUDA(cudaStreamSynchronize(s));
+    const int rb = read_back(&head, mem, sizeof(head), s);
+    if (rb) return rb;
     if (head.bad & (kTcAsymmetric | kTcLoop)) {
         // not a simple undirected graph: Burkhardt's sum (sum ((A * A) .* A)) / 6 as it stands
         gbk_matrix C = nullptr;
