@@ -188,6 +188,11 @@ template <typename T> struct Semiring<GBK_PLUS_ONE, T> {
     __device__ static T mul(T, T) { return T(1); }
 };
 
+// Semirings whose mul reads A_ij; the others' kernels leave the values unread.
+template <int SR>
+constexpr bool kUsesValues = SR != GBK_PLUS_SECOND && SR != GBK_STRUCTURAL_BOOL && SR != GBK_MIN_SECOND &&
+                             SR != GBK_PLUS_ONE;
+
 // Host-side probe add(3, 5) used by the reference to pick the SpMSpV kernel
 // (src/backend/spmspv/spmspv.h:117-146): 8 -> atomic add, 1 -> store 1,
 // otherwise a generic read-modify-write.

@@ -3,8 +3,8 @@
 // Rows are grouped by degree at build time (a stable sort by bin keeps rows
 // ascending inside a bin):
 //   bin 0           empty rows                      one thread per row
-//   bins G=1..32    degree in (G/2, G]              G lanes per row (shuffle reduce)
-//   warp bin        degree 33..kSplitNnz            one warp per row, 4 loads in flight per lane
+//   bins G=1..32    degree in (G, 2G]               G lanes per row, 2 entries per lane at once
+//   warp bin        degree 65..kSplitNnz            one warp per row, 4 loads in flight per lane
 //   split bin       degree > kSplitNnz              the row is cut into kSplitNnz chunks,
 //                                                   one warp per chunk, partials folded
 //                                                   in chunk order by a small fix-up kernel
@@ -20,6 +20,7 @@
 // degree-matched lane groups.
 #include <cub/cub.cuh>
 
+#include <algorithm>
 #include <vector>
 
 #include "common.cuh"
@@ -30,10 +31,12 @@ namespace gbk {
 namespace {
 
 constexpr int kBinThreads = 256;
+constexpr int kBinWarps = kBinThreads / 32;
 #ifndef GBK_SPLIT_NNZ
 #define GBK_SPLIT_NNZ 2048
 #endif
 constexpr int kSplitNnz = GBK_SPLIT_NNZ;
+constexpr int kLaneNnz = 2;  // entries per lane of a group
 // bins: 0 empty, 1..6 -> G = 1,2,4,8,16,32, 7 warp, 8 split
 constexpr int kNumBins = 9;
 constexpr int kBinWarp = 7;
@@ -41,14 +44,9 @@ constexpr int kBinSplit = 8;
 
 __host__ __device__ inline int bin_of_degree(int d) {
     if (d == 0) return 0;
-    if (d <= 1) return 1;
-    if (d <= 2) return 2;
-    if (d <= 4) return 3;
-    if (d <= 8) return 4;
-    if (d <= 16) return 5;
-    if (d <= 32) return 6;
-    if (d <= kSplitNnz) return kBinWarp;
-    return kBinSplit;
+    for (int b = 1, g = 1; b < kBinWarp; ++b, g *= 2)
+        if (d <= kLaneNnz * g) return b;
+    return d <= kSplitNnz ? kBinWarp : kBinSplit;
 }
 
 struct BinTable {
@@ -56,6 +54,7 @@ struct BinTable {
     int32_t block_end[kNumBins];
     int32_t item_start[kNumBins];       // first item of the bin in perm (split bin: chunk table)
     int32_t items[kNumBins];            // rows (or chunks) in the bin
+    int32_t warp_rows[kNumBins];        // rows per warp (group bins; at most 32)
 };
 
 template <typename T>
@@ -67,37 +66,79 @@ __device__ __forceinline__ void write_out(T* y, int64_t r, T v, int accum, const
     y[r] = (accum == GBK_OP_SECOND) ? v : binop<T>(accum, y[r], v);
 }
 
+// One warp per warp_rows (at most 32) rows of a group bin.  The lanes read the
+// rows' ids, masks and bounds, one row each; the rows inside the mask are then
+// worked on 32 / G at a time, each by G lanes that load their 2 entries of it
+// together.  What bounds short rows is the chain id -> mask -> bounds ->
+// entries -> x, not the bytes: two entries a lane halve the warps that go
+// through it, and a warp of up to 32 rows pays the first three links once and
+// nothing for a row outside the mask.  Min-plus over 1,000,003 uniform rows of
+// about 16, a third of them selected: 185 -> 43 us (one entry a lane 50, four
+// 39); R-MAT 2^20 masked 60 -> 39 (four: 37); plus-times over 300,001 uniform
+// rows 27 -> 17; R-MAT 2^18, 4 M entries, 22.9 -> 22.7.  Four entries a lane
+// lose on R-MAT's many rows of a few entries (2^18 24.9, 2^17 masked 20.8
+// against 18.6), whose loads then spread over four times the sectors.
 template <int SR, typename T, int G>
 __device__ __forceinline__ void rows_by_group(const BinTable& bt, int bin, int lb, const int32_t* __restrict__ ptr,
                                               const int32_t* __restrict__ idx, const T* __restrict__ val,
                                               const int32_t* __restrict__ perm, const T* __restrict__ x,
                                               T* __restrict__ y, int accum, const void* mask, int mdt, int mmode) {
     using S = Semiring<SR, T>;
-    const int sub = threadIdx.x % G;
-    const int64_t k = (int64_t)lb * (kBinThreads / G) + threadIdx.x / G;
-    const bool live = k < bt.items[bin];
-    int32_t r = 0;
-    T acc = S::identity();
-    bool skip = !live;
-    if (live) {
-        r = perm[bt.item_start[bin] + k];
-        if (mask && !mask_selects(mask, mdt, mmode, r)) skip = true;
-        if (!skip) {
-            const uint64_t pol = policy_evict_last();
-            const int32_t b = ld_stream(ptr + r), e = ld_stream(ptr + r + 1);
-            for (int32_t q = b + sub; q < e; q += G)
-                acc = S::add(acc, S::mul(ld_stream(val + q), ld_keep(x + ld_stream(idx + q), pol)));
-        }
+    constexpr unsigned kFull = 0xffffffffu;
+    const int lane = threadIdx.x & 31, sub = lane % G;
+    const int32_t wr = bt.warp_rows[bin];
+    const int64_t k0 = ((int64_t)lb * kBinWarps + (threadIdx.x >> 5)) * wr;
+    const int64_t left = bt.items[bin] - k0;
+    if (left <= 0) return;  // the whole warp leaves together
+    int32_t r = 0, b = 0, e = 0;
+    T old = T(0);
+    bool in = false;
+    if (lane < wr && lane < left) {
+        r = perm[bt.item_start[bin] + k0 + lane];
+        b = __ldg(ptr + r);
+        e = __ldg(ptr + r + 1);
+        in = !mask || mask_selects(mask, mdt, mmode, r);
+        if (!in) y[r] = T(0);  // outside the mask (spmv_csr.h:324-327)
+        else if (accum != GBK_OP_SECOND) old = y[r];
     }
-    if (G > 1) {
+    const unsigned rows = __ballot_sync(kFull, in);
+    const int nrows = __popc(rows);
+    // lane i: the lane that holds the i-th row inside the mask
+    int from = lane;
+    if (mask) {
+        from = 0;
 #pragma unroll
-        for (int off = G / 2; off > 0; off >>= 1) acc = S::add(acc, __shfl_xor_sync(0xffffffffu, acc, off, G));
+        for (int w = 16; w >= 1; w >>= 1)
+            if (__popc(rows & ((1u << (from + w)) - 1u)) <= lane) from += w;
     }
-    if (live && sub == 0) {
-        if (skip)
-            y[r] = T(0);  // outside the mask (spmv_csr.h:324-327)
-        else
-            y[r] = (accum == GBK_OP_SECOND) ? acc : binop<T>(accum, y[r], acc);
+    const uint64_t pol = policy_evict_last();
+    for (int i0 = 0; i0 < nrows; i0 += 32 / G) {
+        const int i = i0 + lane / G;
+        const int src = __shfl_sync(kFull, from, i & 31);
+        const int32_t row = __shfl_sync(kFull, r, src), rb = __shfl_sync(kFull, b, src);
+        const int32_t re = __shfl_sync(kFull, e, src);
+        const T row_old = __shfl_sync(kFull, old, src);
+        const bool live = i < nrows;
+        int32_t c[kLaneNnz];
+        T a[kLaneNnz];
+#pragma unroll
+        for (int u = 0; u < kLaneNnz; ++u) {
+            const int32_t q = rb + sub + u * G;
+            const bool in_row = live && q < re;
+            c[u] = in_row ? ld_stream(idx + q) : -1;
+            if constexpr (kUsesValues<SR>) a[u] = in_row ? ld_stream(val + q) : T(0);
+            else a[u] = T(0);
+        }
+        T xv[kLaneNnz];
+#pragma unroll
+        for (int u = 0; u < kLaneNnz; ++u) xv[u] = c[u] >= 0 ? ld_keep(x + c[u], pol) : T(0);
+        T acc = S::identity();
+#pragma unroll
+        for (int u = 0; u < kLaneNnz; ++u)
+            if (c[u] >= 0) acc = S::add(acc, S::mul(a[u], xv[u]));
+#pragma unroll
+        for (int off = G / 2; off > 0; off >>= 1) acc = S::add(acc, __shfl_xor_sync(kFull, acc, off, G));
+        if (live && sub == 0) y[row] = (accum == GBK_OP_SECOND) ? acc : binop<T>(accum, row_old, acc);
     }
 }
 
@@ -117,7 +158,7 @@ __device__ __forceinline__ T warp_range(int32_t b, int32_t e, const int32_t* __r
     for (int u = 0; u < U; u++) {
         const int32_t p = q + 32 * u;
         c[u] = p < e ? ld_stream(idx + p) : -1;
-        a[u] = p < e ? ld_stream(val + p) : T(0);
+        a[u] = kUsesValues<SR> && p < e ? ld_stream(val + p) : T(0);
     }
     for (; q < e; q += 32 * U) {
         int cn[U];
@@ -126,7 +167,7 @@ __device__ __forceinline__ T warp_range(int32_t b, int32_t e, const int32_t* __r
         for (int u = 0; u < U; u++) {
             const int32_t p = q + 32 * (U + u);
             cn[u] = p < e ? ld_stream(idx + p) : -1;
-            an[u] = p < e ? ld_stream(val + p) : T(0);
+            an[u] = kUsesValues<SR> && p < e ? ld_stream(val + p) : T(0);
         }
 #pragma unroll
         for (int u = 0; u < U; u++)
@@ -222,9 +263,39 @@ __global__ void k_bin_keys(const int32_t* ptr, int64_t n, uint32_t* key, int32_t
 
 }  // namespace
 
+namespace {
+
+// CTAs per bin, heaviest bin first; returns their number.
+int64_t place_blocks(BinTable& bt, bool masked) {
+    // A warp takes more than the rows it works on at once where the bin would
+    // fill the machine's warps more than once (300,001 uniform rows: 16.6 us,
+    // 18.7 where it would twice), and with a mask four times as many, as most
+    // rows may be outside it.
+    const int64_t warps = (int64_t)num_sms() * 64;
+    int64_t blk = 0;
+    for (int b = kNumBins - 1; b >= 0; b--) {
+        int64_t per_block = b == 0 ? kBinThreads : kBinWarps;
+        bt.warp_rows[b] = 1;
+        if (b >= 1 && b < kBinWarp) {
+            const int at_once = 32 >> (b - 1);
+            int rows = at_once;
+            while (rows < 32 && bt.items[b] > rows * warps) rows *= 2;
+            if (masked) rows = std::min(32, 4 * rows);
+            bt.warp_rows[b] = rows;
+            per_block = (int64_t)kBinWarps * rows;
+        }
+        bt.block_start[b] = (int32_t)blk;
+        blk += (bt.items[b] + per_block - 1) / per_block;
+        bt.block_end[b] = (int32_t)blk;
+    }
+    return blk;
+}
+
+}  // namespace
+
 // Binned layout of one CSR orientation (held by the view's owner).
 struct RowBins {
-    BinTable bt{};
+    BinTable bt[2]{};                // without and with a mask
     int32_t* perm = nullptr;         // rows sorted by bin (stable)
     int32_t* chunk_row = nullptr;    // split chunks: row and first entry
     int32_t* chunk_beg = nullptr;
@@ -232,7 +303,7 @@ struct RowBins {
     int32_t* split_first = nullptr;
     int64_t nsplit = 0, nchunks = 0;
     void* chunk_out = nullptr;
-    int64_t blocks = 0;
+    int64_t blocks[2] = {0, 0};
 };
 
 void free_bins(RowBins* b) {
@@ -303,21 +374,16 @@ int build_bins(const CsrView& v, int elem_bytes, RowBins** out, cudaStream_t s) 
         GBK_CUDA(cudaMemcpyAsync(rb->split_first, split_first.data(), 4 * (rb->nsplit + 1), cudaMemcpyHostToDevice, s));
         GBK_CUDA(cudaStreamSynchronize(s));
     }
-    // block table: items in bin order (perm is sorted by bin), CTAs heaviest bin first
-    int64_t blk = 0, item = 0;
-    const int per_block[kNumBins] = {kBinThreads, kBinThreads, kBinThreads / 2, kBinThreads / 4, kBinThreads / 8,
-                                     kBinThreads / 16, kBinThreads / 32, kBinThreads / 32, kBinThreads / 32};
+    // items in bin order (perm is sorted by bin)
+    int64_t item = 0;
     for (int b = 0; b < kNumBins; b++) {
-        rb->bt.item_start[b] = (int32_t)item;
-        rb->bt.items[b] = (int32_t)((b == kBinSplit) ? rb->nchunks : counts[b]);
+        for (int m = 0; m < 2; m++) {
+            rb->bt[m].item_start[b] = (int32_t)item;
+            rb->bt[m].items[b] = (int32_t)((b == kBinSplit) ? rb->nchunks : counts[b]);
+        }
         item += counts[b];
     }
-    for (int b = kNumBins - 1; b >= 0; b--) {
-        rb->bt.block_start[b] = (int32_t)blk;
-        blk += (rb->bt.items[b] + per_block[b] - 1) / per_block[b];
-        rb->bt.block_end[b] = (int32_t)blk;
-    }
-    rb->blocks = blk;
+    for (int m = 0; m < 2; m++) rb->blocks[m] = place_blocks(rb->bt[m], m == 1);
     *out = rb;
     return GBK_SUCCESS;
 }
@@ -325,9 +391,10 @@ int build_bins(const CsrView& v, int elem_bytes, RowBins** out, cudaStream_t s) 
 template <int SR, typename T>
 int spmv_binned_t(const RowBins* rb, const CsrView& v, int accum, const T* x, T* y, const void* mask, int mdt,
                   int mmode, cudaStream_t s) {
-    if (rb->blocks > 0) {
-        k_spmv_binned<SR, T><<<(unsigned)rb->blocks, kBinThreads, 0, s>>>(
-            rb->bt, v.ptr, v.idx, (const T*)v.val, rb->perm, rb->chunk_row, rb->chunk_beg, x, y, accum, mask, mdt,
+    const int m = mask ? 1 : 0;
+    if (rb->blocks[m] > 0) {
+        k_spmv_binned<SR, T><<<(unsigned)rb->blocks[m], kBinThreads, 0, s>>>(
+            rb->bt[m], v.ptr, v.idx, (const T*)v.val, rb->perm, rb->chunk_row, rb->chunk_beg, x, y, accum, mask, mdt,
             mmode, (T*)rb->chunk_out);
         GBK_LAUNCHED();
     }
