@@ -270,65 +270,6 @@ __device__ __forceinline__ bool mask_selects(const void* m, int dtype, int mode,
     return mode == GBK_MASK_STR_COMP ? !v : v;
 }
 
-// ----------------------------------------------------------------------------
-// searches in ascending offsets by a whole warp
-
-// Largest k in [0, nf) with offs[k] <= e (offs ascending, offs[nf] > e),
-// found by the whole warp: each round the 31 lanes probe 31 evenly spaced
-// entries of the open range and a ballot keeps the sub-range, so a frontier
-// of n entries takes about log32(n) rounds of one load each.
-__device__ __forceinline__ int64_t warp_find_entry(const int32_t* __restrict__ offs, int64_t nf, int64_t e,
-                                                   int lane) {
-    int64_t lo = 0, hi = nf;  // offs[lo] <= e < offs[hi] (offs[nf] = E > e)
-    while (hi - lo > 1) {
-        const int64_t span = hi - lo;
-        const int64_t p = lo + (span * (lane + 1) + 31) / 32;  // lanes 0..30 probe inside (lo, hi]
-        const bool le = lane < 31 && p < hi && offs[p] <= e;
-        const unsigned bal = __ballot_sync(0xffffffffu, le);
-        const int c = __popc(bal);  // a prefix of the lanes (offs ascends)
-        const int64_t p_c = __shfl_sync(0xffffffffu, p, c < 31 ? c : 30);
-        const int64_t p_last = __shfl_sync(0xffffffffu, p, c > 0 ? c - 1 : 0);
-        if (c > 0) lo = p_last;
-        if (c < 31) hi = p_c;
-    }
-    return lo;
-}
-
-// Entry k (offs[k] <= e < offs[k + 1]) of every lane's element e = e0 + lane,
-// given that k0 is the entry of e0: the lanes load the next 32 boundaries and
-// each finds its own by a 5-step search over them in registers.  E = offs[nf];
-// lanes with e >= E get no entry (an undefined k).  *start = offs[k].
-__device__ __forceinline__ int64_t warp_entry_of(const int32_t* __restrict__ offs, int64_t nf, int64_t k0, int64_t e,
-                                                 int64_t E, int lane, int32_t* start = nullptr) {
-    constexpr unsigned kAllLanes = 0xffffffffu;
-    const int64_t kb = k0 + 1 + lane;  // boundary of entry k0 + 1 + lane (E past the last entry)
-    const int32_t b = kb <= nf ? offs[kb] : (int32_t)E;
-    // cnt = boundaries <= e among the 32 (they ascend with the lane)
-    int cnt = 0;
-#pragma unroll
-    for (int step = 16; step >= 1; step >>= 1) {
-        const int32_t bv = __shfl_sync(kAllLanes, b, cnt + step - 1);
-        if (bv <= e) cnt += step;
-    }
-    const int32_t b31 = __shfl_sync(kAllLanes, b, 31);
-    const int32_t prev = __shfl_sync(kAllLanes, b, cnt > 0 ? cnt - 1 : 0);
-    if (e < E && cnt == 31 && b31 <= e) {
-        // more than 32 entries end before this element (empty ones): search on
-        int64_t lo = k0 + 32, hi = nf;
-        while (hi - lo > 1) {
-            const int64_t mid = (lo + hi) >> 1;
-            if (offs[mid] <= e)
-                lo = mid;
-            else
-                hi = mid;
-        }
-        if (start) *start = offs[lo];
-        return lo;
-    }
-    if (start) *start = cnt > 0 ? prev : offs[k0];
-    return k0 + cnt;
-}
-
 template <typename T> constexpr int dtype_of_t();
 template <> constexpr int dtype_of_t<float>() { return GBK_F32; }
 template <> constexpr int dtype_of_t<int32_t>() { return GBK_I32; }

@@ -5,6 +5,8 @@
 #include <stdint.h>
 #include <stddef.h>
 
+#include <vector>
+
 #include "gbk.h"
 
 namespace gbk {
@@ -104,6 +106,29 @@ int ensure_csc(gbk_matrix A, cudaStream_t s);
 void free_single_cache(gbk_matrix A);
 void free_batches(gbk_matrix A);  // batched.cu
 int build_tiles(CsrView& v, int elem_bytes, cudaStream_t s);
+
+// Device scratch from the stream-ordered pool (reused across calls), freed
+// on the stream on every exit.
+struct StreamScratch {
+    cudaStream_t s;
+    std::vector<void*> p;
+    explicit StreamScratch(cudaStream_t st) : s(st) {}
+    StreamScratch(const StreamScratch&) = delete;
+    ~StreamScratch() {
+        for (void* q : p) cudaFreeAsync(q, s);
+    }
+    template <typename X>
+    int get(X** x, size_t bytes) {
+        void* q = nullptr;
+        if (cudaMallocAsync(&q, bytes < 16 ? 16 : bytes, s) != cudaSuccess) {
+            cudaGetLastError();
+            return GBK_OUT_OF_MEMORY;
+        }
+        p.push_back(q);
+        *x = (X*)q;
+        return GBK_SUCCESS;
+    }
+};
 void free_view(CsrView& v);
 int free_formats(gbk_matrix A);
 

@@ -4,20 +4,19 @@
 // (src/backend/spmspv/spmspv.h:103-158, spmspv_atomics.h:5-170): for every
 // frontier entry (i, x_i) scatter mul(A, x_i) into y.  The reference gives
 // each OpenMP thread frontier vertices and updates y with `omp atomic`,
-// plain stores or an `omp critical` section per edge.  Here the work unit is
-// an edge: a scan of the frontier degrees turns the frontier into one flat
-// edge range, cut into warp tiles of 256 consecutive edges, so a hub vertex
-// is spread over many warps.  Per tile the warp finds the frontier entry of
-// the tile's first edge (a 32-way search, one load per lane per round); per
-// 32-edge sub-tile the lanes load the next 32 entry boundaries and each lane
-// finds its own entry by a 5-step search over those boundaries in registers
-// (shuffles).  Updates are warp-aggregated:
-// lanes whose edges hit the same output element (match-any on the index)
-// combine their values with the semiring's add in a tree over the group,
-// and one lane per group issues the atomic (add; min on integers, a CAS loop
-// on floats).  Or-monoids store 1 without an atomic, as the reference does.
-#include <cub/cub.cuh>
-
+// plain stores or an `omp critical` section per edge.  Here a warp takes 8 or
+// 32 frontier entries and spreads the edges of their rows under kHeavyRow
+// entries over its lanes; longer rows are cut into kPiece-entry pieces that a
+// second kernel hands out one per warp, so a hub is spread over many warps.
+// (The first form scanned the frontier's degrees, copied y and masked it in a
+// pass of its own: nine operations on the stream and four allocations, which
+// took longer than the pushes.  Or-and from 3 % of the vertices of an R-MAT
+// graph of 2^20, masked: 56 -> 25 us.)  Updates are
+// warp-aggregated: lanes whose edges hit the same output element (match-any on
+// the index) combine their values with the semiring's add in a tree over the
+// group, and one lane per group issues the atomic (add; min on integers, a CAS
+// loop on floats).  Or-monoids store 1 without an atomic, as the reference
+// does, and read neither values nor frontier values.
 #include "common.cuh"
 #include "internal.h"
 
@@ -38,13 +37,6 @@ __device__ __forceinline__ void atomic_min_val(float* p, float v) {
     }
 }
 
-__global__ void k_frontier_degrees(const int32_t* __restrict__ ptr, const int32_t* __restrict__ ids, int64_t nf,
-                                   int32_t* __restrict__ deg) {
-    int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (k < nf) deg[k] = ptr[ids[k] + 1] - ptr[ids[k]];
-    if (k == nf) deg[k] = 0;
-}
-
 // Bit position of the r-th (0-based) set bit of m (m has more than r bits).
 __device__ __forceinline__ int nth_set_bit(unsigned m, int r) {
     int pos = 0;
@@ -54,79 +46,164 @@ __device__ __forceinline__ int nth_set_bit(unsigned m, int r) {
     return pos;
 }
 
-template <int SR, typename T>
-__device__ __forceinline__ void push_atomic(int probe, T* y, int32_t j, T v) {
-    using S = Semiring<SR, T>;
-    if (probe == 8)
-        atomicAdd(y + j, v);
-    else  // min-monoids (min, first-min, min-plus, min-second, min-noteq)
-        atomic_min_val(y + j, S::add(Lim<T>::max(), v));
+// What a push does to y[j], by the semiring's add(3, 5) (semiring_probe).
+enum { kPushAdd, kPushOne, kPushMin, kPushNothing };
+template <int SR>
+constexpr int push_kind() {
+    if (SR == GBK_PLUS_TIMES || SR == GBK_PLUS_SECOND || SR == GBK_PLUS_ONE) return kPushAdd;
+    if (SR == GBK_LOR_LAND || SR == GBK_STRUCTURAL_BOOL || SR == GBK_CUSTOM_LESS_PLUS) return kPushOne;
+    return SR == GBK_FIRST_WINS ? kPushNothing : kPushMin;  // first(y, m) == y
 }
 
-constexpr int kPushSubTiles = 8;  // 32-edge sub-tiles per warp tile
+constexpr int kHeavyRow = 32;  // rows with at least this many entries are cut into pieces
+constexpr int kPiece = 128;    // entries per piece
 
-// One warp per tile of 256 consecutive frontier edges (grid-stride over
-// tiles; the loops are warp-uniform, so every shuffle sees all 32 lanes).
-// The tile's first entry comes from one warp search; each 32-edge sub-tile
-// starts from the entry of the previous sub-tile's last edge.
+struct PushArgs {
+    const int32_t* ptr;
+    const int32_t* idx;
+    const void* val;
+    const int32_t* ids;
+    const void* xv;
+    int64_t nf;
+    void* y;
+    const void* mask;  // elements outside it are left alone (NULL: none)
+    int mdt, mmode;
+    int take;          // frontier entries per warp
+    int2* pieces;      // (frontier entry, first entry of the row's piece)
+    int32_t* npieces;
+    int32_t room;      // pieces that fit; a row that would pass it is pushed where it stands
+};
+
+// One push per lane: entry pos of the row, frontier value x.
 template <int SR, typename T>
-__global__ void __launch_bounds__(kPushThreads) k_push(const int32_t* __restrict__ ptr,
-                                                       const int32_t* __restrict__ idx, const T* __restrict__ val,
-                                                       const int32_t* __restrict__ ids, const T* __restrict__ xv,
-                                                       int64_t nf, const int32_t* __restrict__ offs, int probe,
-                                                       T* __restrict__ y) {
+__device__ __forceinline__ void push_edge(const PushArgs& a, bool valid, int64_t pos, T x, int lane) {
     using S = Semiring<SR, T>;
     constexpr unsigned kFull = 0xffffffffu;
-    constexpr int64_t kTile = 32 * kPushSubTiles;
-    const int lane = threadIdx.x & 31;
-    const int64_t E = offs[nf];
-    const int64_t ntiles = (E + kTile - 1) / kTile;
-    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t t = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; t < ntiles; t += nwarps) {
-        int64_t k0 = warp_find_entry(offs, nf, t * kTile, lane);
-        for (int sub = 0; sub < kPushSubTiles; ++sub) {
-            const int64_t e0 = t * kTile + 32 * sub;
-            if (e0 >= E) break;
-            const int64_t e = e0 + lane;
-            const bool valid = e < E;
-            int32_t start;
-            const int64_t k = warp_entry_of(offs, nf, k0, e, E, lane, &start);
-            int32_t j = -1 - lane;  // a key no other lane has
-            T m = S::identity();
-            if (valid) {
-                const int32_t src = ids[k];
-                const int64_t pos = ptr[src] + (e - start);
-                j = idx[pos];
-                m = S::mul(val[pos], xv[k]);
-            }
-            if (probe == 1) {
-                if (valid) y[j] = T(1);
-            } else if (SR != GBK_FIRST_WINS) {
-                // first(y, m) == y leaves y unchanged; every other add folds per group
-                const unsigned peers = __match_any_sync(kFull, j);
-                const int rank = __popc(peers & ((1u << lane) - 1u));
-                const int gsize = __popc(peers);
-                T acc = m;
-                for (int st = 1; st < 32; st <<= 1) {
-                    if (!__any_sync(kFull, gsize > st)) break;
-                    const bool take = (rank % (2 * st)) == 0 && rank + st < gsize;
-                    const int from = take ? nth_set_bit(peers, rank + st) : lane;
-                    const T o = __shfl_sync(kFull, acc, from);
-                    if (take) acc = S::add(acc, o);
-                }
-                if (valid && rank == 0) push_atomic<SR, T>(probe, y, j, acc);
-            }
-            // the next sub-tile starts in the entry of this one's last edge
-            // (valid whenever a next sub-tile exists: e0 + 32 < E)
-            k0 = __shfl_sync(kFull, k, 31);
+    T* y = (T*)a.y;
+    int32_t j = -1 - lane;  // a key no other lane has
+    if (valid) {
+        j = __ldg(a.idx + pos);
+        if (a.mask && !mask_selects(a.mask, a.mdt, a.mmode, j)) {
+            valid = false;
+            j = -1 - lane;
+        }
+    }
+    if constexpr (push_kind<SR>() == kPushOne) {
+        if (valid) y[j] = T(1);
+    } else {
+        T acc = S::identity();
+        if (valid) {
+            T v = T(0);
+            if constexpr (kUsesValues<SR>) v = __ldg((const T*)a.val + pos);
+            acc = S::mul(v, x);
+        }
+        const unsigned peers = __match_any_sync(kFull, j);
+        const int rank = __popc(peers & ((1u << lane) - 1u));
+        const int gsize = __popc(peers);
+        for (int st = 1; st < 32; st <<= 1) {
+            if (!__any_sync(kFull, gsize > st)) break;
+            const bool more = (rank % (2 * st)) == 0 && rank + st < gsize;
+            const int from = more ? nth_set_bit(peers, rank + st) : lane;
+            const T o = __shfl_sync(kFull, acc, from);
+            if (more) acc = S::add(acc, o);
+        }
+        if (valid && rank == 0) {
+            if constexpr (push_kind<SR>() == kPushAdd) atomicAdd(y + j, acc);
+            else atomic_min_val(y + j, S::add(Lim<T>::max(), acc));
         }
     }
 }
 
+// Rows under kHeavyRow entries, edge by edge over the warp's lanes; longer
+// ones are listed for k_push_pieces.  Every loop is warp-uniform.
+template <int SR, typename T>
+__global__ void __launch_bounds__(kPushThreads) k_push(PushArgs a) {
+    constexpr unsigned kFull = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const int64_t ngroups = (a.nf + a.take - 1) / a.take;
+    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    for (int64_t g = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; g < ngroups; g += nwarps) {
+        const int64_t k = g * a.take + lane;
+        int32_t beg = 0, deg = 0;
+        T x = T(0);
+        if (lane < a.take && k < a.nf) {
+            const int32_t u = __ldg(a.ids + k);
+            beg = __ldg(a.ptr + u);
+            deg = __ldg(a.ptr + u + 1) - beg;
+            if constexpr (push_kind<SR>() != kPushOne) x = __ldg((const T*)a.xv + k);
+        }
+        bool heavy = deg >= kHeavyRow;
+        if (heavy) {
+            const int32_t np = (deg + kPiece - 1) / kPiece;
+            const int32_t at = atomicAdd(a.npieces, np);
+            if (at >= 0 && at <= a.room - np)
+                for (int32_t i = 0; i < np; ++i) a.pieces[at + i] = make_int2((int32_t)k, beg + i * kPiece);
+            else if (at >= 0 && at < a.room)
+                for (int32_t i = at; i < a.room; ++i) a.pieces[i] = make_int2(-1, 0);
+            // what does not fit is pushed here
+            heavy = at >= 0 && at <= a.room - np;
+        }
+        const int32_t dl = heavy ? 0 : deg;
+        unsigned lone = __ballot_sync(kFull, dl >= kHeavyRow);
+        const int32_t mine = dl >= kHeavyRow ? 0 : dl;
+        int32_t incl = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int32_t up = __shfl_up_sync(kFull, incl, o);
+            if (lane >= o) incl += up;
+        }
+        const int32_t before = incl - mine;
+        const int32_t total = __shfl_sync(kFull, incl, 31);
+        for (int32_t t0 = 0; t0 < total; t0 += 32) {
+            const int32_t t = t0 + lane;
+            // the row of edge t: the first lane whose inclusive count exceeds t
+            int j = 0;
+#pragma unroll
+            for (int st = 16; st; st >>= 1)
+                if (__shfl_sync(kFull, incl, j + st - 1) <= t) j += st;
+            j = min(j, 31);  // lanes past the end
+            const int32_t eb = __shfl_sync(kFull, beg, j), ex = __shfl_sync(kFull, before, j);
+            const T xj = __shfl_sync(kFull, x, j);
+            push_edge<SR, T>(a, t < total, (int64_t)eb + (t - ex), xj, lane);
+        }
+        while (lone) {  // rows whose pieces did not fit
+            const int j = __ffs(lone) - 1;
+            lone &= lone - 1;
+            const int32_t eb = __shfl_sync(kFull, beg, j), d = __shfl_sync(kFull, deg, j);
+            const T xj = __shfl_sync(kFull, x, j);
+            for (int32_t t0 = 0; t0 < d; t0 += 32) push_edge<SR, T>(a, t0 + lane < d, (int64_t)eb + t0 + lane, xj, lane);
+        }
+    }
+}
+
+// The listed pieces, one warp each.
+template <int SR, typename T>
+__global__ void __launch_bounds__(kPushThreads) k_push_pieces(PushArgs a) {
+    const int lane = threadIdx.x & 31;
+    const int32_t listed = *a.npieces;
+    const int64_t np = listed < 0 || listed > a.room ? a.room : listed;
+    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    for (int64_t c = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; c < np; c += nwarps) {
+        const int2 pc = a.pieces[c];
+        if (pc.x < 0) continue;
+        T x = T(0);
+        if constexpr (push_kind<SR>() != kPushOne) x = __ldg((const T*)a.xv + pc.x);
+        const int32_t end = min(pc.y + kPiece, __ldg(a.ptr + __ldg(a.ids + pc.x) + 1));
+#pragma unroll 4
+        for (int32_t e0 = pc.y; e0 < end; e0 += 32) push_edge<SR, T>(a, e0 + lane < end, (int64_t)e0 + lane, x, lane);
+    }
+}
+
+// y = the identity, 0 outside the mask (if any); the old values are kept in
+// `old` (if any) for an accumulator.
 template <typename T>
-__global__ void k_fill_t(T* y, int64_t n, T v) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        y[i] = v;
+__global__ void k_push_begin(T* y, int64_t n, T ident, T* old, const void* m, int mdt, int mmode, int32_t* npieces) {
+    const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (tid == 0) *npieces = 0;
+    for (int64_t i = tid; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        if (old) old[i] = y[i];
+        y[i] = !m || mask_selects(m, mdt, mmode, i) ? ident : T(0);
+    }
 }
 
 // apply_mask (spmspv.h:17-99), dense form (sparse complements are expanded first)
@@ -186,7 +263,6 @@ template <typename T>
 int spmspv_t(int sr, const CsrView& v, int accum, const int32_t* ids, const void* xv, int64_t nf, T* y,
              const gbk_mask* mask, cudaStream_t s) {
     const int64_t n = v.nrows == v.ncols ? v.ncols : v.ncols;  // y is indexed by the pushed-to side
-    const int probe = semiring_probe(sr, 0);
     T ident;
     switch (sr) {
         case GBK_MIN_PLUS:
@@ -198,32 +274,59 @@ int spmspv_t(int sr, const CsrView& v, int accum, const int32_t* ids, const void
         default:
             ident = T(0);
     }
+    // Without an accumulator (second) the mask needs no old values and no pass
+    // of its own: elements outside it are set to 0 at the start and never
+    // pushed to (a list of ids that is not complemented changes nothing).  A
+    // mask that shares memory with y is applied at the end, to the new values.
+    const bool apart = !mask || !mask->dense || (const char*)mask->dense >= (const char*)(y + n) ||
+                       (const char*)mask->dense + dtype_size(mask->dtype) * (size_t)n <= (const char*)y;
+    const bool second = accum == GBK_OP_SECOND && apart;
+    if (second && mask && !mask->dense && mask->mode != GBK_MASK_STR_COMP) mask = nullptr;
+    const int64_t room = nf > 0 ? v.nnz / kHeavyRow + 1 : 0;  // of a frontier without repeats
+    StreamScratch dev(s);
+    PushArgs a{v.ptr, v.idx, v.val, ids, xv, nf, y, nullptr, 0, 0, 0, nullptr, nullptr, 0};
     T* old = nullptr;
-    if (mask) {
-        GBK_CUDA(cudaMallocAsync((void**)&old, sizeof(T) * (n > 0 ? n : 1), s));
-        GBK_CUDA(cudaMemcpyAsync(old, y, sizeof(T) * n, cudaMemcpyDeviceToDevice, s));
+    uint8_t* flag = nullptr;
+    int32_t* mem = nullptr;
+    if (dev.get(&mem, 16 + sizeof(int2) * (size_t)room) || (mask && !second && dev.get(&old, sizeof(T) * (size_t)n)) ||
+        (mask && !mask->dense && mask->mode == GBK_MASK_STR_COMP && dev.get(&flag, (size_t)n))) {
+        set_error("gbk_spmspv: out of device memory");
+        return GBK_OUT_OF_MEMORY;
+    }
+    a.npieces = mem;
+    a.pieces = (int2*)(mem + 4);
+    a.room = (int32_t)room;
+    // a small frontier gets more warps: 8 entries each until they fill the SMs
+    a.take = nf < (int64_t)num_sms() * 64 * 32 ? 8 : 32;
+    if (flag) {
+        GBK_CUDA(cudaMemsetAsync(flag, 0, n, s));
+        if (mask->nvals > 0) {
+            k_mark<<<grid_cap(mask->nvals, 256), 256, 0, s>>>(mask->ids, mask->nvals, flag);
+            GBK_LAUNCHED();
+        }
+    }
+    const void* dmask = !mask ? nullptr : mask->dense ? mask->dense : flag;
+    const int mdt = mask && mask->dense ? mask->dtype : GBK_BOOL, mmode = mask ? mask->mode : 0;
+    if (second) {
+        a.mask = dmask;
+        a.mdt = mdt;
+        a.mmode = mmode;
     }
     if (n > 0) {
-        k_fill_t<T><<<grid_cap(n, 256), 256, 0, s>>>(y, n, ident);
+        k_push_begin<T><<<grid_cap(n, 256), 256, 0, s>>>(y, n, ident, old, a.mask, a.mdt, a.mmode, a.npieces);
         GBK_LAUNCHED();
     }
-    if (nf > 0) {
-        int32_t *deg = nullptr, *offs = nullptr;
-        GBK_CUDA(cudaMallocAsync((void**)&deg, sizeof(int32_t) * (nf + 1), s));
-        GBK_CUDA(cudaMallocAsync((void**)&offs, sizeof(int32_t) * (nf + 1), s));
-        k_frontier_degrees<<<(unsigned)((nf + 1 + 255) / 256), 256, 0, s>>>(v.ptr, ids, nf, deg);
-        GBK_LAUNCHED();
-        size_t tb = 0;
-        cub::DeviceScan::ExclusiveSum(nullptr, tb, deg, offs, (int)(nf + 1), s);
-        void* tmp = nullptr;
-        GBK_CUDA(cudaMallocAsync(&tmp, tb, s));
-        GBK_CUDA(cub::DeviceScan::ExclusiveSum(tmp, tb, deg, offs, (int)(nf + 1), s));
-        count_launch(1);
-        const unsigned grid = (unsigned)num_sms() * 8;
-#define PUSH_CASE(SRV)                                                                                          \
-    case SRV:                                                                                                   \
-        k_push<SRV, T><<<grid, kPushThreads, 0, s>>>(v.ptr, v.idx, (const T*)v.val, ids, (const T*)xv, nf, offs, \
-                                                     probe, y);                                                 \
+    if (nf > 0 && n > 0) {
+        const unsigned grid = grid_cap((nf + a.take - 1) / a.take * 32, kPushThreads);
+        const unsigned pgrid = grid_cap(room * 32, kPushThreads);
+#define PUSH_CASE(SRV)                                                 \
+    case SRV:                                                          \
+        if constexpr (push_kind<SRV>() != kPushNothing) {              \
+            k_push<SRV, T><<<grid, kPushThreads, 0, s>>>(a);           \
+            GBK_LAUNCHED();                                            \
+            k_push_pieces<SRV, T><<<pgrid, kPushThreads, 0, s>>>(a);   \
+            GBK_LAUNCHED();                                            \
+        }                                                              \
         break;
         switch (sr) {
             PUSH_CASE(GBK_PLUS_TIMES)
@@ -242,34 +345,16 @@ int spmspv_t(int sr, const CsrView& v, int accum, const int32_t* ids, const void
                 return GBK_INVALID_VALUE;
         }
 #undef PUSH_CASE
-        GBK_LAUNCHED();
-        cudaFreeAsync(tmp, s);
-        cudaFreeAsync(deg, s);
-        cudaFreeAsync(offs, s);
     }
-    if (mask && n > 0) {
-        if (mask->dense) {
-            k_apply_mask_dense<T><<<grid_cap(n, 256), 256, 0, s>>>(y, old, n, accum, mask->dense, mask->dtype,
-                                                                   mask->mode);
+    if (mask && !second && n > 0) {
+        if (dmask) {
+            k_apply_mask_dense<T><<<grid_cap(n, 256), 256, 0, s>>>(y, old, n, accum, dmask, mdt, mmode);
             GBK_LAUNCHED();
-        } else if (mask->mode == GBK_MASK_STR_COMP) {
-            uint8_t* flag = nullptr;
-            GBK_CUDA(cudaMallocAsync((void**)&flag, n, s));
-            GBK_CUDA(cudaMemsetAsync(flag, 0, n, s));
-            if (mask->nvals > 0) {
-                k_mark<<<grid_cap(mask->nvals, 256), 256, 0, s>>>(mask->ids, mask->nvals, flag);
-                GBK_LAUNCHED();
-            }
-            k_apply_mask_dense<T><<<grid_cap(n, 256), 256, 0, s>>>(y, old, n, accum, flag, GBK_BOOL,
-                                                                   GBK_MASK_STR_COMP);
-            GBK_LAUNCHED();
-            cudaFreeAsync(flag, s);
         } else if (mask->nvals > 0) {
             k_apply_mask_ids<T><<<grid_cap(mask->nvals, 256), 256, 0, s>>>(y, old, mask->ids, mask->nvals, accum);
             GBK_LAUNCHED();
         }
     }
-    if (old) cudaFreeAsync(old, s);
     return GBK_SUCCESS;
 }
 
