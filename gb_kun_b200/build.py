@@ -42,6 +42,7 @@ CU_SOURCES = [
     "single.cu",
     "vector_ops.cu",
     "spgemm.cu",
+    "spgemm_window.cu",
     "tune.cu",
     "noalloc.cu",
     "batched.cu",

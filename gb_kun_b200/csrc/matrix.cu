@@ -73,6 +73,8 @@ int alloc_carries(CsrView& v, int elem_bytes) {
     return GBK_SUCCESS;
 }
 
+constexpr size_t kPoolKeep = 4ull << 30;
+
 int bits_for(int64_t n) {
     int b = 1;
     while ((1LL << b) < n) b++;
@@ -158,6 +160,33 @@ int ensure_csc(gbk_matrix A, cudaStream_t s) {
     return GBK_SUCCESS;
 }
 
+int adopt_csr(gbk_matrix* out, int64_t nrows, int64_t ncols, int64_t nnz, int32_t* ptr, int32_t* idx, void* val,
+              gbk_dtype vtype, cudaStream_t s) {
+    gbk_matrix A = new gbk_matrix_s();
+    cudaGetDevice(&A->device);
+    A->vtype = vtype;
+    A->pooled = true;
+    CsrView& v = A->csr;
+    v.nrows = nrows;
+    v.ncols = ncols;
+    v.nnz = nnz;
+    v.ptr = ptr;
+    v.idx = idx;
+    v.val = val;
+    int rc = build_tiles(v, (int)dtype_size(vtype), s);
+    if (rc == GBK_SUCCESS && cudaStreamSynchronize(s) != cudaSuccess)
+        rc = cuda_fail(cudaGetLastError(), "adopt_csr", __FILE__, __LINE__);
+    if (rc) {
+        v.ptr = v.idx = nullptr;  // the caller's again
+        v.val = nullptr;
+        free_view(v);
+        delete A;
+        return rc;
+    }
+    *out = A;
+    return GBK_SUCCESS;
+}
+
 }  // namespace gbk
 
 using namespace gbk;
@@ -212,10 +241,26 @@ int gbk_matrix_destroy(gbk_matrix A) {
     free_batches(A);
     free_single_cache(A);
     free_formats(A);
+    int current = 0;
+    cudaGetDevice(&current);
+    if (A->pooled) {
+        // unlike cudaMalloc'd arrays, the pool's are freed without waiting for work in flight
+        cudaSetDevice(A->device);
+        cudaDeviceSynchronize();
+        for (void* p : {(void*)A->csr.ptr, (void*)A->csr.idx, A->csr.val}) cudaFreeAsync(p, 0);
+        A->csr.ptr = A->csr.idx = nullptr;
+        A->csr.val = nullptr;
+    }
     free_view(A->csr);
     free_view(A->csc);
     cudaFree(A->xcopy);
     cudaFree(A->coldeg);
+    if (A->pooled) {
+        // results that come and go are served from the pool; beyond this much it is given back
+        cudaMemPool_t pool;
+        if (cudaDeviceGetDefaultMemPool(&pool, A->device) == cudaSuccess) cudaMemPoolTrimTo(pool, kPoolKeep);
+        cudaSetDevice(current);
+    }
     delete A;
     return GBK_SUCCESS;
 }

@@ -186,25 +186,6 @@ __global__ void k_nonzero_flags(const T* __restrict__ v, int64_t n, uint8_t* __r
 
 unsigned nb(int64_t n) { return (unsigned)std::max<int64_t>(1, (n + 255) / 256); }
 
-// Device scratch from the stream-ordered pool (reused across calls), freed
-// on the stream on every exit.
-struct Scratch {
-    cudaStream_t s;
-    std::vector<void*> p;
-    explicit Scratch(cudaStream_t st) : s(st) {}
-    ~Scratch() {
-        for (void* q : p) cudaFreeAsync(q, s);
-    }
-    template <typename X>
-    int get(X** x, size_t bytes) {
-        void* q = nullptr;
-        if (cudaMallocAsync(&q, std::max<size_t>(bytes, 16), s) != cudaSuccess) return GBK_OUT_OF_MEMORY;
-        p.push_back(q);
-        *x = (X*)q;
-        return GBK_SUCCESS;
-    }
-};
-
 // Products per block: keys, values and their sorted copies, about 24 bytes
 // each.  GBK_MXM_BLOCK_PRODUCTS (at least 1) overrides it, so small products
 // can exercise several blocks.
@@ -219,7 +200,7 @@ int64_t block_products() {
 template <int SR, typename T>
 int mxm_unmasked(gbk_matrix* out, const CsrView& a, const CsrView& b, cudaStream_t s) {
     const int64_t n = a.nrows, m = b.ncols, annz = a.nnz;
-    Scratch dev(s);
+    StreamScratch dev(s);
     auto need = [&](int rc) { return rc == GBK_SUCCESS; };
     int64_t* off = nullptr;
     int32_t* arow = nullptr;
@@ -830,7 +811,7 @@ extern "C" int gbk_triangle_count(gbk_matrix A, uint64_t* count, void* stream) {
     // Everything up to the count is queued before the one read-back: the
     // kernels after k_tc_mark look at its verdict on the device.
     const int64_t ntiles = (nnz + kTcTile - 1) / kTcTile;
-    Scratch dev(s);
+    StreamScratch dev(s);
     uint8_t* mem = nullptr;  // bad, class counts, total, then the arrays
     size_t tb = 0;
     cub::DeviceScan::ExclusiveSum(nullptr, tb, (int32_t*)nullptr, (int32_t*)nullptr, ntiles + 1, s);
@@ -974,6 +955,10 @@ extern "C" int gbk_mxm(gbk_matrix* out, gbk_matrix A, gbk_matrix B, gbk_semiring
     GBK_REQUIRE(A->csr.ncols == B->csr.nrows, GBK_DIMENSION_MISMATCH, "gbk_mxm: A is %lldx%lld, B %lldx%lld",
                 (long long)A->csr.nrows, (long long)A->csr.ncols, (long long)B->csr.nrows, (long long)B->csr.ncols);
     cudaStream_t s = (cudaStream_t)stream;
+    bool done = false;
+    // a windowed entry takes 8 bytes of scratch, an expanded product 24
+    const int rc = mxm_window(out, A->csr, B->csr, A->vtype, sr, 3 * block_products(), &done, s);
+    if (rc || done) return rc;
 #define MXM_CASE(SRV)                                                                                 \
     case SRV:                                                                                         \
         return A->vtype == GBK_F32 ? mxm_unmasked<SRV, float>(out, A->csr, B->csr, s)                 \

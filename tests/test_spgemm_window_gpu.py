@@ -1,0 +1,145 @@
+"""gbk_mxm at the edges of its column windows (2,048 columns, at most 64 of them) and for the operands
+that the windows refuse (repeated or unsorted columns, too many columns, too few products a window),
+against sums in numpy: whole numbers, so every order of the sums gives the same value."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+COLS = [1, 31, 2047, 2048, 2049, 4097, 64 * 2048 - 1, 64 * 2048, 64 * 2048 + 1]
+
+
+@pytest.fixture(scope="module")
+def capi():
+    from gb_kun_b200 import capi
+    capi.init(0)
+    return capi
+
+
+def csr(rows, cols, n):
+    ptr = np.zeros(n + 1, np.int64)
+    np.add.at(ptr, rows + 1, 1)
+    return np.cumsum(ptr).astype(np.int32), cols.astype(np.int32)
+
+
+def pattern(rng, n, m, count):
+    """Distinct (row, column) pairs, half of them in the first rows and all columns at both ends."""
+    r = np.minimum(rng.integers(0, n, count), rng.integers(0, n, count) * 4)
+    c = rng.integers(0, m, count)
+    c[:8] = [0, m - 1] * 4
+    key = np.unique(r.astype(np.int64) * m + c)
+    return key // m, key % m
+
+
+def product(ar, ac, av, br, bc, bv, m, sr):
+    """Entries (key, value) of the product from all its terms, zeros dropped."""
+    nb = int(br.max()) + 1
+    order = np.argsort(br, kind="stable")
+    br, bc, bv = br[order], bc[order], bv[order]
+    start = np.searchsorted(br, np.arange(max(nb, int(ac.max()) + 1) + 1))
+    cnt = start[ac + 1] - start[ac]
+    e = np.repeat(np.arange(len(ac)), cnt)
+    f = np.arange(cnt.sum()) - np.repeat(np.cumsum(cnt) - cnt, cnt) + start[ac[e]]
+    key = ar[e].astype(np.int64) * m + bc[f]
+    a, b = av[e].astype(np.int64), bv[f].astype(np.int64)
+    x = {"plus_times": a * b, "plus_second": b, "plus_one": np.ones_like(a), "min_second": b,
+         "min_plus": np.minimum(a + b, np.iinfo(np.int32).max), "lor_land": ((a != 0) & (b != 0)).astype(np.int64)}[sr]
+    keys, inv = np.unique(key, return_inverse=True)
+    if sr.startswith("min"):
+        out = np.full(len(keys), np.iinfo(np.int64).max)
+        np.minimum.at(out, inv, x)
+    else:
+        out = np.zeros(len(keys), np.int64)
+        np.add.at(out, inv, x)
+        if sr == "lor_land":
+            out = np.minimum(out, 1)
+    keep = out != 0
+    return keys[keep], out[keep]
+
+
+def check(capi, A, B, want, m):
+    C = A.mxm(B, semiring=want[0])
+    rp, col, v = C.download_csr()
+    assert (C.n, C.ncols) == (A.n, m)
+    key = np.repeat(np.arange(A.n, dtype=np.int64), np.diff(rp)) * m + col
+    assert np.array_equal(key, want[1])
+    assert np.array_equal(v, want[2].astype(v.dtype))
+
+
+@pytest.mark.parametrize("block", [None, "1", "40009"])
+@pytest.mark.parametrize("sr", ["plus_times", "plus_second", "plus_one", "min_plus", "min_second", "lor_land"])
+@pytest.mark.parametrize("m", COLS)
+def test_windows(capi, monkeypatch, m, sr, block):
+    if block:
+        monkeypatch.setenv("GBK_MXM_BLOCK_PRODUCTS", block)
+    else:
+        monkeypatch.delenv("GBK_MXM_BLOCK_PRODUCTS", raising=False)
+    rng = np.random.default_rng(m)
+    n, k = 61, 47
+    ar, ac = pattern(rng, n, k, 900)
+    br, bc = pattern(rng, k, m, 6000)
+    for dtype in (np.int32, np.float32):
+        av = rng.integers(-3, 4, len(ar)).astype(dtype)
+        bv = rng.integers(-3, 4, len(br)).astype(dtype)
+        if dtype == np.int32 and sr.startswith("min"):
+            av[ar == 5] = 1
+            bv[:] = np.where(rng.random(len(bv)) < 0.3, np.iinfo(np.int32).max, bv)  # reached, and the identity
+        A = capi.Matrix(*csr(ar, ac, n), av, ncols=k)
+        B = capi.Matrix(*csr(br, bc, k), bv, ncols=m)
+        check(capi, A, B, (sr, *product(ar, ac, av, br, bc, bv, m, sr)), m)
+
+
+@pytest.mark.parametrize("sr", ["plus_times", "plus_second", "plus_one", "min_plus", "min_second", "lor_land"])
+@pytest.mark.parametrize("length", [511, 512, 513, 3000])
+def test_hub_rows(capi, monkeypatch, length, sr):
+    # a row that a CTA works on in several rounds, beside short ones
+    monkeypatch.delenv("GBK_MXM_BLOCK_PRODUCTS", raising=False)
+    rng = np.random.default_rng(length)
+    n, k, m = 20, 3000, 2100
+    ar, ac = pattern(rng, n, k, 300)
+    hub = np.sort(rng.permutation(k)[:length])
+    key = np.unique(np.concatenate([ar * k + ac, 7 * k + hub]))
+    ar, ac = key // k, key % k
+    br, bc = pattern(rng, k, m, 200_000)
+    for dtype in (np.int32, np.float32):
+        av, bv = rng.integers(-3, 4, len(ar)).astype(dtype), rng.integers(-3, 4, len(br)).astype(dtype)
+        A = capi.Matrix(*csr(ar, ac, n), av, ncols=k)
+        B = capi.Matrix(*csr(br, bc, k), bv, ncols=m)
+        check(capi, A, B, (sr, *product(ar, ac, av, br, bc, bv, m, sr)), m)
+
+
+@pytest.mark.parametrize("form", ["repeated", "unsorted", "empty"])
+def test_refused_operands(capi, form):
+    rng = np.random.default_rng(3)
+    n, k, m = 40, 30, 5000
+    ar, ac = pattern(rng, n, k, 400)
+    br, bc = pattern(rng, k, m, 3000)
+    if form == "repeated":
+        br, bc = np.concatenate([br, br[::7]]), np.concatenate([bc, bc[::7]])
+        order = np.lexsort((bc, br))
+        br, bc = br[order], bc[order]
+    elif form == "unsorted":
+        order = np.lexsort((-bc, br))
+        br, bc = br[order], bc[order]
+    av = rng.integers(1, 4, len(ar)).astype(np.int32)
+    bv = rng.integers(1, 4, len(br)).astype(np.int32)
+    A = capi.Matrix(*csr(ar, ac, n), av, ncols=k)
+    B = capi.Matrix(*csr(br, bc, k), bv, ncols=m)
+    if form == "empty":
+        E = capi.Matrix(np.zeros(k + 1, np.int32), np.zeros(0, np.int32), np.zeros(0, np.int32), ncols=m)
+        C = A.mxm(E)
+        assert C.nnz == 0 and (C.n, C.ncols) == (n, m)
+        return
+    check(capi, A, B, ("plus_times", *product(ar, ac, av, br, bc, bv, m, "plus_times")), m)
+
+
+def test_infinities_and_nan(capi):
+    # row 0: inf * 0 (NaN, kept) and inf; row 1: 1 * 0 (dropped) and inf - inf; row 2: -inf + inf
+    A = capi.Matrix(np.array([0, 1, 3, 5], np.int32), np.array([0, 0, 1, 1, 2], np.int32),
+                    np.array([np.inf, 1, 1, 1, 1], np.float32), ncols=3)
+    B = capi.Matrix(np.array([0, 2, 3, 4], np.int32), np.array([0, 2500, 2500, 2500], np.int32),
+                    np.array([0, np.inf, -np.inf, np.inf], np.float32), ncols=3000)
+    rp, col, v = A.mxm(B).download_csr()
+    assert rp.tolist() == [0, 2, 3, 4] and col.tolist() == [0, 2500, 2500, 2500]
+    assert np.isnan(v[0]) and v[1] == np.inf and np.isnan(v[2]) and np.isnan(v[3])
