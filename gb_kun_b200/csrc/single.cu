@@ -222,10 +222,39 @@ __device__ __forceinline__ void queue_append(bool found, int32_t v, int32_t* q, 
     if (found) q[base + __popc(m & ((1u << lane) - 1u))] = v;
 }
 
+// The same for U values a lane, with one atomic per warp.
+template <int U>
+__device__ __forceinline__ void queue_append(const bool (&found)[U], const int32_t (&v)[U], int32_t* q,
+                                             int32_t* count) {
+    unsigned m[U];
+    int32_t total = 0;
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+        m[k] = __ballot_sync(kAll, found[k]);
+        total += __popc(m[k]);
+    }
+    if (!total) return;
+    const int lane = threadIdx.x & 31;
+    int32_t base = 0;
+    if (lane == 0) base = atomicAdd(count, total);
+    base = __shfl_sync(kAll, base, 0);
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+        if (found[k]) q[base + __popc(m[k] & ((1u << lane) - 1u))] = v[k];
+        base += __popc(m[k]);
+    }
+}
+
 // The rows of the frontier qc[0, fc): rows under kHeavy entries edge by edge
-// over the warp's lanes (op.edge(valid, value of the row, entry) on every
+// over the warp's lanes (op.edges(valid, value of the row, entry) on every
 // lane), longer rows appended to `chunks` for expand_heavy.  Op::load(u)
-// gives the per-row value passed to op.edge.
+// gives the per-row value passed to op.edges.  Bound by the chain entry ->
+// neighbour's state -> atomic -> queue, so an operator gets kBatch entries a
+// lane at a time and overlaps their chains (four against one:
+// SSSP on R-MAT 2^20 2.44 -> 2.01 ms, on 300,001 uniform vertices 2.21 -> 1.82;
+// BFS on 700,001 uniform vertices 371 -> 298 us, R-MAT 2^21 338 -> 325).
+constexpr int kBatch = 4;
+
 template <class Op>
 __device__ void expand_light(const int32_t* __restrict__ qc, int32_t fc, const int32_t* __restrict__ rp,
                              Chunk* __restrict__ chunks, int32_t* nchunks, Op& op) {
@@ -252,16 +281,27 @@ __device__ void expand_light(const int32_t* __restrict__ qc, int32_t fc, const i
         const int32_t excl = incl - dl;
         const int32_t total = __shfl_sync(kAll, incl, 31);
         const V val = dl > 0 ? op.load(u) : V();
-        for (int32_t t0 = 0; t0 < total; t0 += 32) {
-            const int32_t t = t0 + lane;
-            // the row of edge t: the first lane whose inclusive count exceeds t
-            int j = 0;
-            for (int s = 16; s; s >>= 1)
-                if (__shfl_sync(kAll, incl, j + s - 1) <= t) j += s;
-            j = min(j, 31);  // lanes past the end
-            const int32_t eb = __shfl_sync(kAll, beg, j), ex = __shfl_sync(kAll, excl, j);
-            const V vj = __shfl_sync(kAll, val, j);
-            op.edge(t < total, vj, eb + (t - ex));
+        for (int32_t t0 = 0; t0 < total; t0 += 32 * kBatch) {
+            bool valid[kBatch];
+            V vals[kBatch];
+            int32_t e[kBatch];
+#pragma unroll
+            for (int k = 0; k < kBatch; ++k) {
+                const int32_t t = t0 + 32 * k + lane;
+                valid[k] = t < total;
+                vals[k] = V();
+                e[k] = 0;
+                if (t0 + 32 * k >= total) continue;  // the whole warp
+                // the row of edge t: the first lane whose inclusive count exceeds t
+                int j = 0;
+                for (int s = 16; s; s >>= 1)
+                    if (__shfl_sync(kAll, incl, j + s - 1) <= t) j += s;
+                j = min(j, 31);  // lanes past the end
+                const int32_t eb = __shfl_sync(kAll, beg, j), ex = __shfl_sync(kAll, excl, j);
+                vals[k] = __shfl_sync(kAll, val, j);
+                e[k] = eb + (t - ex);
+            }
+            op.template edges<kBatch>(valid, vals, e);
         }
     }
 }
@@ -275,7 +315,18 @@ __device__ void expand_heavy(const Chunk* __restrict__ chunks, int32_t nch, cons
         const Chunk ch = chunks[c];
         const int32_t end = min(ch.beg + kChunk, rp[ch.u + 1]);
         const typename Op::V val = op.load(ch.u);
-        for (int32_t e0 = ch.beg; e0 < end; e0 += 32) op.edge(e0 + lane < end, val, e0 + lane);
+        for (int32_t e0 = ch.beg; e0 < end; e0 += 32 * kBatch) {
+            bool valid[kBatch];
+            typename Op::V vals[kBatch];
+            int32_t e[kBatch];
+#pragma unroll
+            for (int k = 0; k < kBatch; ++k) {
+                e[k] = e0 + 32 * k + lane;
+                valid[k] = e[k] < end;
+                vals[k] = val;
+            }
+            op.template edges<kBatch>(valid, vals, e);
+        }
     }
 }
 
@@ -326,29 +377,38 @@ struct BfsNext {
     int32_t* qn;
     uint32_t* bn;
     int32_t* ncount;
-    long long edges;
+    long long edges_out;
 
     __device__ V load(int32_t) const { return 0; }
     __device__ __forceinline__ void record(bool found, int32_t v) {
         queue_append(found, v, qn, ncount);
         if (found) {
             atomicOr(bn + (v >> 5), 1u << (v & 31));
-            edges += rp[v + 1] - rp[v];
+            edges_out += rp[v + 1] - rp[v];
         }
     }
-    // top-down: claim an unvisited column
-    __device__ __forceinline__ void edge(bool valid, V, int32_t e) {
-        int32_t v = -1;
-        bool found = false;
-        if (valid) {
-            v = col[e];
-            found = lv[v] == 0 && atomicCAS(lv + v, 0, next) == 0;
-        }
-        record(found, v);
+    // top-down: claim unvisited columns
+    template <int U>
+    __device__ __forceinline__ void edges(const bool (&valid)[U], const V (&)[U], const int32_t (&e)[U]) {
+        int32_t v[U];
+        bool found[U];
+#pragma unroll
+        for (int k = 0; k < U; ++k) v[k] = valid[k] ? __ldg(col + e[k]) : -1;
+#pragma unroll
+        for (int k = 0; k < U; ++k) found[k] = v[k] >= 0 && __ldcg(lv + v[k]) == 0;
+#pragma unroll
+        for (int k = 0; k < U; ++k) found[k] = found[k] && atomicCAS(lv + v[k], 0, next) == 0;
+        queue_append<U>(found, v, qn, ncount);
+#pragma unroll
+        for (int k = 0; k < U; ++k)
+            if (found[k]) {
+                atomicOr(bn + (v[k] >> 5), 1u << (v[k] & 31));
+                edges_out += rp[v[k] + 1] - rp[v[k]];
+            }
     }
     __device__ void flush(long long* total) {
-        for (int o = 16; o; o >>= 1) edges += __shfl_xor_sync(kAll, edges, o);
-        if ((threadIdx.x & 31) == 0 && edges) atomicAdd((unsigned long long*)total, (unsigned long long)edges);
+        for (int o = 16; o; o >>= 1) edges_out += __shfl_xor_sync(kAll, edges_out, o);
+        if ((threadIdx.x & 31) == 0 && edges_out) atomicAdd((unsigned long long*)total, (unsigned long long)edges_out);
     }
 };
 
@@ -378,12 +438,12 @@ __global__ void __launch_bounds__(kT) k_bfs1_light(Bfs1Bufs b, Bfs1State* st) {
             const int32_t beg = un ? b.crp[v] : 0, deg = un ? b.crp[v + 1] - beg : 0;
             bool found = false;
             if (deg < kHeavy)
-                for (int32_t e = beg; e < beg + deg; ++e) {
-                    const int32_t u = b.crow[e];
-                    if ((bc[u >> 5] >> (u & 31)) & 1u) {
-                        found = true;
-                        break;
-                    }
+                for (int32_t e = beg; e < beg + deg && !found; e += kBatch) {
+                    int32_t u[kBatch];  // neighbouring entries: mostly one sector
+#pragma unroll
+                    for (int k = 0; k < kBatch; ++k) u[k] = e + k < beg + deg ? __ldg(b.crow + e + k) : -1;
+#pragma unroll
+                    for (int k = 0; k < kBatch; ++k) found |= u[k] >= 0 && ((bc[u[k] >> 5] >> (u[k] & 31)) & 1u);
                 }
             unsigned hubs = __ballot_sync(kAll, deg >= kHeavy);
             while (hubs) {
@@ -551,21 +611,28 @@ struct SsspRelax {
     bool use_far;
 
     __device__ V load(int32_t u) const { return __ldcg(dist + u); }
-    __device__ __forceinline__ void edge(bool valid, V du, int32_t e) {
-        int32_t v = -1;
-        bool near = false, pile = false;
-        if (valid) {
-            v = col[e];
-            const T nd = elem_add(du, w[e]);
-            if (nd < __ldcg(dist + v) && atomic_min_improves(dist + v, nd)) {
-                if (!use_far || nd < thr)
-                    near = test_and_set(bn, v);  // queued once per round
-                else
-                    pile = test_and_set(fbm, v);  // in the pile once
-            }
+    template <int U>
+    __device__ __forceinline__ void edges(const bool (&valid)[U], const V (&du)[U], const int32_t (&e)[U]) {
+        int32_t v[U];
+        T nd[U];
+        bool better[U], near[U], pile[U];
+#pragma unroll
+        for (int k = 0; k < U; ++k) {
+            v[k] = valid[k] ? __ldg(col + e[k]) : -1;
+            nd[k] = valid[k] ? elem_add(du[k], __ldg(w + e[k])) : du[k];
         }
-        queue_append(near, v, qn, ncount);
-        queue_append(pile, v, far, farcount);
+#pragma unroll
+        for (int k = 0; k < U; ++k) better[k] = v[k] >= 0 && nd[k] < __ldcg(dist + v[k]);
+#pragma unroll
+        for (int k = 0; k < U; ++k) better[k] = better[k] && atomic_min_improves(dist + v[k], nd[k]);
+#pragma unroll
+        for (int k = 0; k < U; ++k) {
+            const bool is_near = !use_far || nd[k] < thr;
+            near[k] = better[k] && is_near && test_and_set(bn, v[k]);  // queued once per round
+            pile[k] = better[k] && !is_near && test_and_set(fbm, v[k]);  // in the pile once
+        }
+        queue_append<U>(near, v, qn, ncount);
+        queue_append<U>(pile, v, far, farcount);
     }
 };
 
