@@ -10,7 +10,8 @@
 //
 // Unmasked SpGEMM C = A (+.x) B replaces SpMSpM_unmasked_ikj
 // (src/backend/spmspm/spmspm_hash_based_gustavson.h:9-148, a hash map per
-// row of C) by expand-sort-compress in row blocks: every product
+// row of C) by sums in column windows (spgemm_window.cu) and, for the operands
+// those refuse, by expand-sort-compress in row blocks: every product
 // A_ik * B_kj is written with its (i, j) key (one thread per product, found
 // by binary search over the per-entry product offsets), the block is radix
 // sorted by key, equal keys are reduced with the semiring's add, and sums
