@@ -429,9 +429,13 @@ struct Owned {
     }
 };
 
-// A (row of A, window) pair costs about as much as a step of 32 products.
-bool window_pays(int64_t annz, int nw, unsigned long long products) {
-    return (unsigned long long)annz * nw <= 4 * products + 65536;
+// An (entry of A, window) pair costs about as much as a step of 32 products, and
+// the tables of B's parts and of the tasks must not outgrow what the expansion
+// would hold (a hypersparse A or B has far more rows than products).
+bool window_pays(const CsrView& a, const CsrView& b, int nw, unsigned long long products) {
+    const unsigned long long most = 4 * products + 65536;
+    return (unsigned long long)a.nnz * nw <= most && (unsigned long long)a.nrows * nw <= most &&
+           (unsigned long long)b.nrows * (nw + 1) <= most;
 }
 
 template <int SR, typename T>
@@ -452,17 +456,15 @@ int window_t(gbk_matrix* out, const CsrView& a, const CsrView& b, int64_t block_
     WindowHead head;
     GBK_CUDA(cudaMemcpyAsync(&head, d_head, sizeof(head), cudaMemcpyDeviceToHost, s));
     GBK_CUDA(cudaStreamSynchronize(s));
-    if (head.drops != head.row_drops || !window_pays(a.nnz, nw, head.products)) return GBK_SUCCESS;
+    if (head.drops != head.row_drops || !window_pays(a, b, nw, head.products)) return GBK_SUCCESS;
     // the parts of B's rows and the tasks' room
     int32_t *seg = nullptr, *order = nullptr;
     int64_t *room = nullptr, *off = nullptr;
     uint8_t* cls = nullptr;
     if (dev.get(&seg, 4 * (size_t)b.nrows * (nw + 1)) || dev.get(&order, 4 * (size_t)ntasks) ||
         dev.get(&room, 8 * (size_t)(ntasks + 1)) || dev.get(&off, 8 * (size_t)(ntasks + 1)) ||
-        dev.get(&cls, (size_t)ntasks)) {
-        set_error("gbk_mxm: out of device memory");
-        return GBK_OUT_OF_MEMORY;
-    }
+        dev.get(&cls, (size_t)ntasks))
+        return GBK_SUCCESS;  // not done: the expansion may still fit
     k_win_bounds<<<nb(b.nrows * (nw + 1)), 256, 0, s>>>(b.ptr, b.idx, b.nrows * (nw + 1), nw, seg);
     GBK_LAUNCHED();
     k_win_tasks<<<(unsigned)std::min<int64_t>((ntasks + 7) / 8, (int64_t)num_sms() * 8), 256, 0, s>>>(
@@ -514,10 +516,8 @@ int window_t(gbk_matrix* out, const CsrView& a, const CsrView& b, int64_t block_
     int64_t* count = room;  // the rooms have been scanned
     int64_t* fin = nullptr;
     if (dev.get(&tcol, 4 * (size_t)max_room) || dev.get(&tval, sizeof(T) * (size_t)max_room) ||
-        dev.get(&fin, 8 * (size_t)(ntasks + 1))) {
-        set_error("gbk_mxm: out of device memory for %lld entries per block", (long long)max_room);
-        return GBK_OUT_OF_MEMORY;
-    }
+        dev.get(&fin, 8 * (size_t)(ntasks + 1)))
+        return GBK_SUCCESS;  // not done
     const int smem = (int)(sizeof(T) + (flagged<SR>() ? 1 : 0)) * kWin * kWinWarps;
     GBK_CUDA(cudaFuncSetAttribute(k_win_numeric<SR, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     const int per_sm = flagged<SR>() ? 2 : 3;

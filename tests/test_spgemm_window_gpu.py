@@ -109,10 +109,10 @@ def test_hub_rows(capi, monkeypatch, length, sr):
         check(capi, A, B, (sr, *product(ar, ac, av, br, bc, bv, m, sr)), m)
 
 
-@pytest.mark.parametrize("form", ["repeated", "unsorted", "empty"])
+@pytest.mark.parametrize("form", ["repeated", "unsorted", "empty", "tall"])
 def test_refused_operands(capi, form):
     rng = np.random.default_rng(3)
-    n, k, m = 40, 30, 5000
+    n, k, m = (40, 200_000, 64 * 2048) if form == "tall" else (40, 30, 5000)  # tall: far more rows than products
     ar, ac = pattern(rng, n, k, 400)
     br, bc = pattern(rng, k, m, 3000)
     if form == "repeated":
