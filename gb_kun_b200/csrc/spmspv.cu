@@ -17,6 +17,8 @@
 // group, and one lane per group issues the atomic (add; min on integers, a CAS
 // loop on floats).  Or-monoids store 1 without an atomic, as the reference
 // does, and read neither values nor frontier values.
+#include <algorithm>
+
 #include "common.cuh"
 #include "internal.h"
 
@@ -282,13 +284,16 @@ int spmspv_t(int sr, const CsrView& v, int accum, const int32_t* ids, const void
                        (const char*)mask->dense + dtype_size(mask->dtype) * (size_t)n <= (const char*)y;
     const bool second = accum == GBK_OP_SECOND && apart;
     if (second && mask && !mask->dense && mask->mode != GBK_MASK_STR_COMP) mask = nullptr;
-    const int64_t room = nf > 0 ? v.nnz / kHeavyRow + 1 : 0;  // of a frontier without repeats
+    // pieces of a frontier without repeats; a small frontier over a huge matrix
+    // gets room for its likely ones, and none at all when memory is short
+    int64_t room = nf > 0 ? std::min<int64_t>(v.nnz / kHeavyRow + 1, (1 << 20) + 64 * nf) : 0;
     StreamScratch dev(s);
     PushArgs a{v.ptr, v.idx, v.val, ids, xv, nf, y, nullptr, 0, 0, 0, nullptr, nullptr, 0};
     T* old = nullptr;
     uint8_t* flag = nullptr;
     int32_t* mem = nullptr;
-    if (dev.get(&mem, 16 + sizeof(int2) * (size_t)room) || (mask && !second && dev.get(&old, sizeof(T) * (size_t)n)) ||
+    if (dev.get(&mem, 16 + sizeof(int2) * (size_t)room)) room = 0;
+    if ((room == 0 && !mem && dev.get(&mem, 16)) || (mask && !second && dev.get(&old, sizeof(T) * (size_t)n)) ||
         (mask && !mask->dense && mask->mode == GBK_MASK_STR_COMP && dev.get(&flag, (size_t)n))) {
         set_error("gbk_spmspv: out of device memory");
         return GBK_OUT_OF_MEMORY;
