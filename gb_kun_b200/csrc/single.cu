@@ -251,8 +251,8 @@ __device__ __forceinline__ void queue_append(const bool (&found)[U], const int32
 // gives the per-row value passed to op.edges.  Bound by the chain entry ->
 // neighbour's state -> atomic -> queue, so an operator gets kBatch entries a
 // lane at a time and overlaps their chains (four against one:
-// SSSP on R-MAT 2^20 2.44 -> 2.01 ms, on 300,001 uniform vertices 2.21 -> 1.82;
-// BFS on 700,001 uniform vertices 371 -> 298 us, R-MAT 2^21 338 -> 325).
+// SSSP on R-MAT 2^20 2.32 -> 1.90 ms, on 300,001 uniform vertices 2.21 -> 1.82;
+// BFS on 700,001 uniform vertices 371 -> 298 us, R-MAT 2^21 353 -> 319).
 constexpr int kBatch = 4;
 
 template <class Op>
