@@ -160,8 +160,22 @@ __global__ void __launch_bounds__(256) k_win_tasks(const int32_t* __restrict__ a
     if (threadIdx.x < kClasses && h[threadIdx.x]) atomicAdd(hist + threadIdx.x, h[threadIdx.x]);
 }
 
-// Tasks with products, heaviest class first (inside a class in any order).
-__global__ void __launch_bounds__(256) k_win_order(const uint8_t* __restrict__ cls, int64_t ntasks,
+// Number of tasks per class of a block's tasks.
+__global__ void __launch_bounds__(256) k_win_classes(const uint8_t* __restrict__ cls, int64_t ntasks,
+                                                     int32_t* __restrict__ hist) {
+    __shared__ int32_t h[kClasses];
+    if (threadIdx.x < kClasses) h[threadIdx.x] = 0;
+    __syncthreads();
+    const int64_t nth = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < ntasks; t += nth)
+        if (cls[t] != 255) atomicAdd(h + cls[t], 1);
+    __syncthreads();
+    if (threadIdx.x < kClasses && h[threadIdx.x]) atomicAdd(hist + threadIdx.x, h[threadIdx.x]);
+}
+
+// The tasks [task0, task0 + ntasks) with products, heaviest class first (inside
+// a class in any order); cls and order from task0 on.
+__global__ void __launch_bounds__(256) k_win_order(const uint8_t* __restrict__ cls, int64_t task0, int64_t ntasks,
                                                    const int32_t* __restrict__ hist, int32_t* __restrict__ cursor,
                                                    int32_t* __restrict__ order) {
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -176,7 +190,7 @@ __global__ void __launch_bounds__(256) k_win_order(const uint8_t* __restrict__ c
         at += atomicAdd(cursor + c, __popc(peers));
     }
     at = __shfl_sync(peers, at, lead);
-    order[at + __popc(peers & ((1u << lane) - 1u))] = (int32_t)t;
+    order[at + __popc(peers & ((1u << lane) - 1u))] = (int32_t)(task0 + t);
 }
 
 struct WindowArgs {
@@ -188,9 +202,9 @@ struct WindowArgs {
     const int32_t* seg;
     int nw;
     int64_t task0;            // first task of the block
-    const int32_t* order;     // tasks to run (NULL: task0 .. task0 + ntasks - 1)
+    const int32_t* order;     // tasks to run
     int64_t nheavy;           // the first ones, a CTA each
-    int64_t ntasks;
+    int64_t ntasks;           // their number
     const int64_t* off;       // room before each task
     int64_t off0;             // room before the block
     int32_t* tcol;            // the tasks' entries, each task's at off[task] - off0
@@ -371,7 +385,7 @@ __global__ void __launch_bounds__(32 * kWinWarps, 3) k_win_numeric(WindowArgs g)
         if (lane == 0) i = atomicAdd(g.next + 1, 1ull);
         i = __shfl_sync(kAll, i, 0) + g.nheavy;
         if ((long long)i >= g.ntasks) break;
-        const int64_t task = g.order ? (int64_t)g.order[i] : g.task0 + (int64_t)i;
+        const int64_t task = g.order[i];
         const int64_t row = task / g.nw;
         const int w = (int)(task - row * g.nw);
         window_sums<SR, T>(g, w, g.aptr[row], g.aptr[row + 1], acc, seen, lane);
@@ -470,7 +484,7 @@ int window_t(gbk_matrix* out, const CsrView& a, const CsrView& b, int64_t block_
     k_win_tasks<<<(unsigned)std::min<int64_t>((ntasks + 7) / 8, (int64_t)num_sms() * 8), 256, 0, s>>>(
         a.ptr, a.idx, seg, ntasks, nw, m, room, cls, d_hist);
     GBK_LAUNCHED();
-    k_win_order<<<nb(ntasks), 256, 0, s>>>(cls, ntasks, d_hist, d_cursor, order);
+    k_win_order<<<nb(ntasks), 256, 0, s>>>(cls, 0, ntasks, d_hist, d_cursor, order);
     GBK_LAUNCHED();
     size_t tb = 0;
     cub::DeviceScan::ExclusiveSum(nullptr, tb, room, off, ntasks + 1, s);
@@ -479,15 +493,10 @@ int window_t(gbk_matrix* out, const CsrView& a, const CsrView& b, int64_t block_
     GBK_CUDA(cub::DeviceScan::ExclusiveSum(tmp, tb, room, off, ntasks + 1, s));
     count_launch(1);
     int64_t total_room = 0;
-    int32_t hist[kClasses];
+    std::vector<int32_t> hist(kClasses);  // tasks per class of each block
     GBK_CUDA(cudaMemcpyAsync(&total_room, off + ntasks, 8, cudaMemcpyDeviceToHost, s));
-    GBK_CUDA(cudaMemcpyAsync(hist, d_hist, sizeof(hist), cudaMemcpyDeviceToHost, s));
+    GBK_CUDA(cudaMemcpyAsync(hist.data(), d_hist, 4 * kClasses, cudaMemcpyDeviceToHost, s));
     GBK_CUDA(cudaStreamSynchronize(s));
-    int64_t nrun = 0, nheavy = 0;
-    for (int c = 0; c < kClasses; ++c) {
-        nrun += hist[c];
-        if (c <= kHeavyClass) nheavy += hist[c];
-    }
     // blocks of whole rows with room for at most block_entries entries (a single row may exceed it)
     std::vector<int64_t> cuts{0, n}, hroff{0, total_room};  // cut rows and the room before them
     if (total_room > block_entries) {
@@ -509,6 +518,23 @@ int window_t(gbk_matrix* out, const CsrView& a, const CsrView& b, int64_t block_
         }
     }
     const size_t nblocks = cuts.size() - 1;
+    if (nblocks > 1) {  // each block's tasks in an order of their own
+        int32_t* d_bhist = nullptr;  // per block: tasks per class, then cursors
+        const size_t bytes = 4 * 2 * kClasses * nblocks;
+        if (dev.get(&d_bhist, bytes)) return GBK_SUCCESS;  // not done
+        GBK_CUDA(cudaMemsetAsync(d_bhist, 0, bytes, s));
+        for (size_t c = 0; c < nblocks; ++c) {
+            const int64_t t0 = cuts[c] * nw, nt = (cuts[c + 1] - cuts[c]) * nw;
+            int32_t* h = d_bhist + 2 * kClasses * c;
+            k_win_classes<<<(unsigned)std::min<int64_t>(nb(nt), (int64_t)num_sms() * 8), 256, 0, s>>>(cls + t0, nt, h);
+            GBK_LAUNCHED();
+            k_win_order<<<nb(nt), 256, 0, s>>>(cls + t0, t0, nt, h, h + kClasses, order + t0);
+            GBK_LAUNCHED();
+        }
+        hist.resize(2 * kClasses * nblocks);
+        GBK_CUDA(cudaMemcpyAsync(hist.data(), d_bhist, bytes, cudaMemcpyDeviceToHost, s));
+        GBK_CUDA(cudaStreamSynchronize(s));
+    }
     int64_t max_room = 0;
     for (size_t c = 0; c < nblocks; ++c) max_room = std::max(max_room, hroff[c + 1] - hroff[c]);
     int32_t* tcol = nullptr;
@@ -529,10 +555,14 @@ int window_t(gbk_matrix* out, const CsrView& a, const CsrView& b, int64_t block_
     int64_t total = 0;
     for (size_t c = 0; c < nblocks; ++c) {
         const int64_t t0 = cuts[c] * nw, nt = (cuts[c + 1] - cuts[c]) * nw;
-        const int64_t run = nblocks == 1 ? nrun : nt;
+        int64_t run = 0, nheavy = 0;
+        for (int k = 0; k < kClasses; ++k) {
+            run += hist[2 * kClasses * c + k];
+            if (k <= kHeavyClass) nheavy += hist[2 * kClasses * c + k];
+        }
         GBK_CUDA(cudaMemsetAsync(count, 0, 8 * (size_t)(nt + 1), s));
         GBK_CUDA(cudaMemsetAsync(d_next, 0, 16, s));
-        WindowArgs g{a.ptr, a.idx, a.val, b.idx, b.val, seg, nw, t0, nblocks == 1 ? order : nullptr, nblocks == 1 ? nheavy : 0, run,
+        WindowArgs g{a.ptr, a.idx, a.val, b.idx, b.val, seg, nw, t0, order + t0, nheavy, run,
                      off, hroff[c], tcol, tval, count, d_next};
         if (run > 0) {
             const int64_t ctas = std::min<int64_t>(std::max<int64_t>((run + kWinWarps - 1) / kWinWarps, g.nheavy),

@@ -143,3 +143,32 @@ def test_infinities_and_nan(capi):
     rp, col, v = A.mxm(B).download_csr()
     assert rp.tolist() == [0, 2, 3, 4] and col.tolist() == [0, 2500, 2500, 2500]
     assert np.isnan(v[0]) and v[1] == np.inf and np.isnan(v[2]) and np.isnan(v[3])
+
+
+def dense_rows(rng, rows, length, m):
+    """A with `length` entries in every row, B with all of `m` columns, of random floats in [0, 1)."""
+    ptr = np.arange(0, (rows + 1) * length, length).astype(np.int32)
+    col = np.tile(np.arange(length), rows).astype(np.int32)
+    bptr = np.arange(0, (length + 1) * m, m).astype(np.int32)
+    bcol = np.tile(np.arange(m), length).astype(np.int32)
+    return (ptr, col, rng.random(rows * length).astype(np.float32)), (bptr, bcol, rng.random(length * m).astype(np.float32))
+
+
+@pytest.mark.parametrize("blocks", [1, 5])
+@pytest.mark.parametrize("m,length", [(300, 4000), (2100, 700)])
+def test_float_sums(capi, monkeypatch, m, length, blocks):
+    # Products rounded to 32 bits, their sums in 64: each product of non-negative terms and the final rounding
+    # add at most 2^-24 of the sum.  With 32-bit sums of thousands of terms: 8e-7 in blocks, before these had
+    # windows of 4,096 and more products worked on by whole CTAs.
+    rows = 20
+    rng = np.random.default_rng(m)
+    (ap, ac, av), (bp, bc, bv) = dense_rows(rng, rows, length, m)
+    monkeypatch.delenv("GBK_MXM_BLOCK_PRODUCTS", raising=False)
+    if blocks > 1:  # a block has room for three entries per product allowed
+        monkeypatch.setenv("GBK_MXM_BLOCK_PRODUCTS", str(rows * m // (3 * blocks)))
+    C = capi.Matrix(ap, ac, av, ncols=length).mxm(capi.Matrix(bp, bc, bv, ncols=m))
+    rp, col, v = C.download_csr()
+    assert rp.tolist() == list(range(0, (rows + 1) * m, m)) and np.array_equal(col, np.tile(np.arange(m), rows))
+    want = av.reshape(rows, length).astype(np.float64) @ bv.reshape(length, m).astype(np.float64)
+    err = np.linalg.norm(v.reshape(rows, m) - want) / np.linalg.norm(want)
+    assert err <= 2.0 ** -23
