@@ -1,5 +1,6 @@
 // Unmasked SpGEMM C = A (+.x) B in column windows: one warp (for many products a
-// CTA) per (row of C, window of kWin columns), the window's sums in shared memory.
+// CTA) per (row of C, window of 1,280 or 2,048 columns), the window's sums in shared
+// memory.
 //
 // The warp walks the entries A_ik of its row in order; of every row k of B it
 // takes the part inside its window (the parts' bounds are tabulated per call)
@@ -17,9 +18,9 @@
 // done and the caller expands and sorts the products.
 //
 // A A of an undirected R-MAT graph of 2^14 vertices, 157 M products, 46 M
-// entries: 1.2 ms on the device, where a call took 11.7 ms by expansion and
-// sorting, which move every product through memory several times; what is left
-// is the sums (0.84 ms) and the result's move to its place (0.24 ms).
+// entries: 1.3 ms a call, where it took 11.7 ms by expansion and sorting, which
+// move every product through memory several times; what is left is the sums
+// (0.84 ms) and the result's move to its place (0.26 ms).
 #include <cub/cub.cuh>
 
 #include <algorithm>
@@ -32,10 +33,7 @@ namespace gbk {
 
 namespace {
 
-constexpr int kWin = 2048;       // columns per window: 8 KB of sums per warp, 24 warps on an SM
-constexpr int kWinWarps = 8;     // warps per CTA
-constexpr int kMaxWindows = 64;  // B of up to 131,072 columns
-constexpr int kSteps = 8;        // 32-entry steps of B a warp loads before it adds the first
+constexpr int64_t kMaxColumns = 131072;  // of B
 constexpr unsigned kAll = 0xffffffffu;
 
 // Semirings whose identity may also be a sum (min over values that reach the
@@ -50,8 +48,27 @@ constexpr bool flagged() {
 template <int SR>
 constexpr bool kReadsB = SR != GBK_PLUS_ONE;
 
+// Float sums are formed in 64 bits: a column's sum has as many terms as A's row
+// has entries at most, and 32-bit sums in order lose more than the expansion's
+// (terms of [0, 1): 6.1e-8 from the 64-bit sums at 16 terms, 7.9e-7 at 4,000;
+// 5.2e-8 and 5.4e-8 by expansion).  Their windows are narrower, so that 21 warps
+// fit an SM.  A A in ms, R-MAT 2^14 | 2^15 | 2^12 | uniform 2^14, 16 entries a row:
+// 1,280 columns, 3 warps a CTA 1.32 | 4.5 | 0.32 | 0.71; 1,024 columns (27 warps)
+// 1.36 | 4.7 | 0.33 | 0.71; 2,048 (12 warps) 1.66 | 5.6 | 0.31 | 0.89; 7 warps a CTA
+// 1.47 | 4.9 | 0.34 | 0.72; 32-bit sums, 2,048 columns, 24 warps 1.37 | 4.8 | 0.30 | 0.58.
+template <int SR, typename T>
+struct Shape {
+    static constexpr bool kWide = std::is_same<T, float>::value &&
+                                  (SR == GBK_PLUS_TIMES || SR == GBK_PLUS_SECOND || SR == GBK_PLUS_ONE);
+    using Sum = std::conditional_t<kWide, double, T>;
+    static constexpr int kCols = kWide ? 1280 : 2048;  // columns per window
+    static constexpr int kWarps = kWide ? 3 : 8;       // per CTA
+    static constexpr int kSteps = kWide ? 6 : 8;       // 32-entry steps of B a warp loads before it adds the first
+    static constexpr int kCtas = kWide ? 7 : flagged<SR>() ? 2 : 3;  // on an SM
+    static constexpr int kSmem = (int)(sizeof(Sum) + (flagged<SR>() ? 1 : 0)) * kCols * kWarps;
+};
+
 constexpr int kHeavyClass = 31 - 12;  // tasks of 2^12 products or more are worked on by a whole CTA
-constexpr int kRound = 64;            // entries of A per warp and round of such a task
 
 struct WindowHead {
     unsigned long long products;
@@ -100,13 +117,13 @@ __global__ void __launch_bounds__(256) k_win_head(const int32_t* __restrict__ ai
 
 // seg[k * (nw + 1) + w]: first entry of B's row k in window w or later.
 __global__ void __launch_bounds__(256) k_win_bounds(const int32_t* __restrict__ bptr, const int32_t* __restrict__ bidx,
-                                                    int64_t total, int nw, int32_t* __restrict__ seg) {
+                                                    int64_t total, int nw, int cols, int32_t* __restrict__ seg) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= total) return;
     const int64_t k = i / (nw + 1);
     const int w = (int)(i - k * (nw + 1));
     int32_t lo = bptr[k], hi = bptr[k + 1];
-    const int32_t col = w * kWin;  // below 2^31: at most kMaxWindows windows
+    const int32_t col = w * cols;  // at most kMaxColumns and a window
     if (w == 0) hi = lo;
     if (w == nw) lo = hi;
     while (lo < hi) {
@@ -128,7 +145,7 @@ __device__ __forceinline__ int task_class(long long products) {  // heaviest fir
 // Per task (row, window): its products, bounded by the window's columns
 // (room[task]; room[ntasks] = 0), and the number of tasks per class.
 __global__ void __launch_bounds__(256) k_win_tasks(const int32_t* __restrict__ aptr, const int32_t* __restrict__ aidx,
-                                                   const int32_t* __restrict__ seg, int64_t ntasks, int nw, int64_t m,
+                                                   const int32_t* __restrict__ seg, int64_t ntasks, int nw, int cols, int64_t m,
                                                    int64_t* __restrict__ room, uint8_t* __restrict__ cls,
                                                    int32_t* __restrict__ hist) {
     __shared__ int32_t h[kClasses];
@@ -137,8 +154,7 @@ __global__ void __launch_bounds__(256) k_win_tasks(const int32_t* __restrict__ a
     const int lane = threadIdx.x & 31;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     for (int64_t t = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < ntasks; t += nwarps) {
-        const int64_t row = t / nw;
-        const int w = (int)(t - row * nw);
+        const int32_t row = (int32_t)t / nw, w = (int32_t)t - row * nw;  // tasks are int32
         long long sum = 0;
         const int32_t a1 = aptr[row + 1];
         for (int32_t e = aptr[row] + lane; e < a1; e += 32) {
@@ -148,7 +164,7 @@ __global__ void __launch_bounds__(256) k_win_tasks(const int32_t* __restrict__ a
 #pragma unroll
         for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(kAll, sum, o);
         if (lane == 0) {
-            const long long width = m - (int64_t)w * kWin < kWin ? m - (int64_t)w * kWin : kWin;
+            const long long width = m - (int64_t)w * cols < cols ? m - (int64_t)w * cols : cols;
             room[t] = sum < width ? sum : width;
             const int c = sum > 0 ? task_class(sum) : 255;
             cls[t] = (uint8_t)c;
@@ -215,13 +231,15 @@ struct WindowArgs {
 
 // A warp's sums of one window over the entries [a0, a1) of a row of A.
 template <int SR, typename T>
-__device__ __forceinline__ void window_sums(const WindowArgs& g, int w, int32_t a0, int32_t a1, T* acc, uint8_t* seen,
-                                            int lane) {
+__device__ __forceinline__ void window_sums(const WindowArgs& g, int w, int32_t a0, int32_t a1,
+                                            typename Shape<SR, T>::Sum* acc, uint8_t* seen, int lane) {
     using S = Semiring<SR, T>;
+    using Sum = typename Shape<SR, T>::Sum;
+    constexpr int kSteps = Shape<SR, T>::kSteps;
     const T* __restrict__ aval = (const T*)g.aval;
     const T* __restrict__ bval = (const T*)g.bval;
     const int32_t* __restrict__ bidx = g.bidx;
-    const int32_t col0 = w * kWin;
+    const int32_t col0 = w * Shape<SR, T>::kCols;
     const int32_t* __restrict__ seg = g.seg + w;
     for (; a0 < a1; a0 += 32) {
         int32_t sb = 0, se = 0;
@@ -261,8 +279,10 @@ __device__ __forceinline__ void window_sums(const WindowArgs& g, int w, int32_t 
                     if constexpr (flagged<SR>()) {
                         acc[q] = seen[q] ? S::add(acc[q], x) : x;
                         seen[q] = 1;
-                    } else {
+                    } else if constexpr (std::is_same<Sum, T>::value) {
                         acc[q] = S::add(acc[q], x);
+                    } else {
+                        acc[q] += (Sum)x;
                     }
                 }
                 __syncwarp();  // the next step may meet the same columns in other lanes
@@ -273,25 +293,36 @@ __device__ __forceinline__ void window_sums(const WindowArgs& g, int w, int32_t 
 
 // The window's sums in column order to the task's room, cleared behind the scan.
 template <int SR, typename T>
-__device__ __forceinline__ void window_out(const WindowArgs& g, int64_t task, int w, T* acc, uint8_t* seen, int lane) {
+__device__ __forceinline__ void window_out(const WindowArgs& g, int64_t task, int w, typename Shape<SR, T>::Sum* acc,
+                                           uint8_t* seen, int lane) {
     int64_t at = g.off[task] - g.off0;
     const int64_t first = at;
     T* tval = (T*)g.tval;
-    for (int q = lane; q < kWin; q += 32) {
-        const T v = acc[q];
-        bool keep = v != T(0);
-        if constexpr (flagged<SR>()) {
-            keep = keep && seen[q];
-            seen[q] = 0;
+    constexpr int kAhead = 4;  // loads in flight
+    static_assert(Shape<SR, T>::kCols % (32 * kAhead) == 0, "the scan takes 128 columns at a time");
+    for (int q0 = lane; q0 < Shape<SR, T>::kCols; q0 += 32 * kAhead) {
+        T v[kAhead];
+        bool keep[kAhead];
+#pragma unroll
+        for (int k = 0; k < kAhead; ++k) {
+            v[k] = (T)acc[q0 + 32 * k];
+            keep[k] = v[k] != T(0);
+            if constexpr (flagged<SR>()) keep[k] = keep[k] && seen[q0 + 32 * k];
         }
-        acc[q] = Semiring<SR, T>::identity();
-        const unsigned bal = __ballot_sync(kAll, keep);
-        if (keep) {
-            const int64_t o = at + __popc(bal & ((1u << lane) - 1u));
-            g.tcol[o] = w * kWin + q;
-            tval[o] = v;
+#pragma unroll
+        for (int k = 0; k < kAhead; ++k) {
+            const int q = q0 + 32 * k;
+            if constexpr (flagged<SR>()) seen[q] = 0;
+            acc[q] = Semiring<SR, T>::identity();
+            const unsigned bal = __ballot_sync(kAll, keep[k]);
+            if (!bal) continue;
+            if (keep[k]) {
+                const int64_t o = at + __popc(bal & ((1u << lane) - 1u));
+                g.tcol[o] = w * Shape<SR, T>::kCols + q;
+                tval[o] = v[k];
+            }
+            at += __popc(bal);
         }
-        at += __popc(bal);
     }
     __syncwarp();
     if (lane == 0) g.count[task - g.task0] = at - first;
@@ -300,28 +331,22 @@ __device__ __forceinline__ void window_out(const WindowArgs& g, int64_t task, in
 // Bound by the steps (a 32-entry piece of a row of B: two coalesced loads, a
 // shared-memory load, add and store), about 30 instructions each; kSteps of
 // them are loaded ahead, across the ends of B's rows, to cover L2's latency.
-// A heavy task is worked on by a whole CTA: in each round every warp adds up to
-// kRound entries of A in a window of its own, and each thread then folds the
-// eight sums of its eight columns into totals in registers, in order.  (With a
-// warp each, the hub rows' windows held the kernel for 1.6 ms on an R-MAT graph
-// of 2^14 vertices, now 0.84.)  Float sums are totalled in 64 bits, so a sum of
-// thousands of products, which lie in the heavy tasks, is rounded over short
-// runs only: that product is 3.2e-8 from its 64-bit sums, 9.5e-8 with 32-bit
-// totals, and 5.5e-8 by the expansion.
+// A heavy task is worked on by a whole CTA: its warps take the row's entries
+// 32 at a time in turn, each into a window of its own, and at the end each
+// thread adds up the sums of its columns in the order of the warps.
 template <int SR, typename T>
-__global__ void __launch_bounds__(32 * kWinWarps, 3) k_win_numeric(WindowArgs g) {
+__global__ void __launch_bounds__(32 * Shape<SR, T>::kWarps, Shape<SR, T>::kCtas) k_win_numeric(WindowArgs g) {
     using S = Semiring<SR, T>;
-    constexpr bool kSum = SR == GBK_PLUS_TIMES || SR == GBK_PLUS_SECOND || SR == GBK_PLUS_ONE;
-    using Total = std::conditional_t<kSum && std::is_same<T, float>::value, double, T>;
-    constexpr int kColumns = kWin / (32 * kWinWarps);
+    using Sum = typename Shape<SR, T>::Sum;
+    constexpr int kCols = Shape<SR, T>::kCols, kWarps = Shape<SR, T>::kWarps;
     extern __shared__ uint8_t smem[];
     __shared__ unsigned long long s_next;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    T* const all = (T*)smem;
-    uint8_t* const all_seen = smem + sizeof(T) * kWin * kWinWarps;  // flagged semirings only
-    T* acc = all + warp * kWin;
-    uint8_t* seen = all_seen + warp * kWin;
-    for (int i = lane; i < kWin; i += 32) {
+    Sum* const all = (Sum*)smem;
+    uint8_t* const all_seen = smem + sizeof(Sum) * kCols * kWarps;  // flagged semirings only
+    Sum* acc = all + warp * kCols;
+    uint8_t* seen = all_seen + warp * kCols;
+    for (int i = lane; i < kCols; i += 32) {
         acc[i] = S::identity();
         if constexpr (flagged<SR>()) seen[i] = 0;
     }
@@ -332,49 +357,33 @@ __global__ void __launch_bounds__(32 * kWinWarps, 3) k_win_numeric(WindowArgs g)
             if (threadIdx.x == 0) s_next = atomicAdd(g.next, 1ull);
             __syncthreads();
             if ((long long)s_next >= g.nheavy) break;
-            const int64_t task = g.order[s_next];
-            const int64_t row = task / g.nw;
-            const int w = (int)(task - row * g.nw);
+            const int32_t task = g.order[s_next];
+            const int32_t row = task / g.nw, w = task - row * g.nw;
             const int32_t a0 = g.aptr[row], a1 = g.aptr[row + 1];
-            const int32_t per = min(kRound, (a1 - a0 + kWinWarps - 1) / kWinWarps);
-            Total tot[kColumns];
-            bool any[kColumns];
+            const int32_t per = min(32, (a1 - a0 + kWarps - 1) / kWarps);  // entries of A per warp and turn
+            for (int64_t from = (int64_t)a0 + warp * per; from < a1; from += kWarps * per)
+                window_sums<SR, T>(g, w, (int32_t)from, (int32_t)(from + per < a1 ? from + per : a1), acc, seen, lane);
+            __syncthreads();
+            for (int q = threadIdx.x; q < kCols; q += 32 * kWarps) {
+                Sum tot = S::identity();
+                bool any = false;
 #pragma unroll
-            for (int k = 0; k < kColumns; ++k) {
-                tot[k] = Total(S::identity());
-                any[k] = false;
-            }
-            for (int64_t base = a0; base < a1; base += (int64_t)kWinWarps * per) {
-                const int64_t from = base + (int64_t)warp * per;
-                if (from < a1)
-                    window_sums<SR, T>(g, w, (int32_t)from, (int32_t)(from + per < a1 ? from + per : a1), acc, seen, lane);
-                __syncthreads();
-#pragma unroll
-                for (int k = 0; k < kColumns; ++k) {
-                    const int q = threadIdx.x + k * 32 * kWinWarps;
-#pragma unroll
-                    for (int i = 0; i < kWinWarps; ++i) {
-                        const T part = all[i * kWin + q];
-                        all[i * kWin + q] = S::identity();
-                        if constexpr (flagged<SR>()) {
-                            if (!all_seen[i * kWin + q]) continue;
-                            all_seen[i * kWin + q] = 0;
-                            tot[k] = any[k] ? S::add(tot[k], part) : part;
-                            any[k] = true;
-                        } else if constexpr (std::is_same<Total, T>::value) {
-                            tot[k] = S::add(tot[k], part);
-                        } else {
-                            tot[k] += (Total)part;
-                        }
+                for (int i = 0; i < kWarps; ++i) {
+                    const Sum part = all[i * kCols + q];
+                    all[i * kCols + q] = S::identity();
+                    if constexpr (flagged<SR>()) {
+                        if (!all_seen[i * kCols + q]) continue;
+                        all_seen[i * kCols + q] = 0;
+                        tot = any ? S::add(tot, part) : part;
+                        any = true;
+                    } else if constexpr (std::is_same<Sum, T>::value) {
+                        tot = S::add(tot, part);
+                    } else {
+                        tot += part;
                     }
                 }
-                __syncthreads();
-            }
-#pragma unroll
-            for (int k = 0; k < kColumns; ++k) {
-                const int q = threadIdx.x + k * 32 * kWinWarps;
-                all[q] = (T)tot[k];
-                if constexpr (flagged<SR>()) all_seen[q] = any[k];
+                all[q] = tot;
+                if constexpr (flagged<SR>()) all_seen[q] = any;
             }
             __syncthreads();
             if (warp == 0) window_out<SR, T>(g, task, w, acc, seen, lane);
@@ -385,9 +394,8 @@ __global__ void __launch_bounds__(32 * kWinWarps, 3) k_win_numeric(WindowArgs g)
         if (lane == 0) i = atomicAdd(g.next + 1, 1ull);
         i = __shfl_sync(kAll, i, 0) + g.nheavy;
         if ((long long)i >= g.ntasks) break;
-        const int64_t task = g.order[i];
-        const int64_t row = task / g.nw;
-        const int w = (int)(task - row * g.nw);
+        const int32_t task = g.order[i];
+        const int32_t row = task / g.nw, w = task - row * g.nw;
         window_sums<SR, T>(g, w, g.aptr[row], g.aptr[row + 1], acc, seen, lane);
         __syncwarp();
         window_out<SR, T>(g, task, w, acc, seen, lane);
@@ -443,10 +451,11 @@ struct Owned {
     }
 };
 
-// An (entry of A, window) pair costs about as much as a step of 32 products, and
-// the tables of B's parts and of the tasks must not outgrow what the expansion
+// An (entry of A, window of 2,048 columns) pair costs about as much as a step of 32
+// products, and the tables of B's parts and of the tasks must not outgrow what the expansion
 // would hold (a hypersparse A or B has far more rows than products).
-bool window_pays(const CsrView& a, const CsrView& b, int nw, unsigned long long products) {
+bool window_pays(const CsrView& a, const CsrView& b, unsigned long long products) {
+    const int64_t nw = (b.ncols + 2047) / 2048;
     const unsigned long long most = 4 * products + 65536;
     return (unsigned long long)a.nnz * nw <= most && (unsigned long long)a.nrows * nw <= most &&
            (unsigned long long)b.nrows * (nw + 1) <= most;
@@ -455,8 +464,10 @@ bool window_pays(const CsrView& a, const CsrView& b, int nw, unsigned long long 
 template <int SR, typename T>
 int window_t(gbk_matrix* out, const CsrView& a, const CsrView& b, int64_t block_entries, bool* done, cudaStream_t s) {
     const int64_t n = a.nrows, m = b.ncols;
-    const int nw = (int)((m + kWin - 1) / kWin);
+    using Sh = Shape<SR, T>;
+    const int nw = (int)((m + Sh::kCols - 1) / Sh::kCols);
     const int64_t ntasks = n * nw;
+    if (ntasks >= INT32_MAX) return GBK_SUCCESS;  // tasks are int32
     StreamScratch dev(s);
     WindowHead* d_head = nullptr;
     if (dev.get(&d_head, 512)) return GBK_OUT_OF_MEMORY;
@@ -470,7 +481,7 @@ int window_t(gbk_matrix* out, const CsrView& a, const CsrView& b, int64_t block_
     WindowHead head;
     GBK_CUDA(cudaMemcpyAsync(&head, d_head, sizeof(head), cudaMemcpyDeviceToHost, s));
     GBK_CUDA(cudaStreamSynchronize(s));
-    if (head.drops != head.row_drops || !window_pays(a, b, nw, head.products)) return GBK_SUCCESS;
+    if (head.drops != head.row_drops || !window_pays(a, b, head.products)) return GBK_SUCCESS;
     // the parts of B's rows and the tasks' room
     int32_t *seg = nullptr, *order = nullptr;
     int64_t *room = nullptr, *off = nullptr;
@@ -479,10 +490,10 @@ int window_t(gbk_matrix* out, const CsrView& a, const CsrView& b, int64_t block_
         dev.get(&room, 8 * (size_t)(ntasks + 1)) || dev.get(&off, 8 * (size_t)(ntasks + 1)) ||
         dev.get(&cls, (size_t)ntasks))
         return GBK_SUCCESS;  // not done: the expansion may still fit
-    k_win_bounds<<<nb(b.nrows * (nw + 1)), 256, 0, s>>>(b.ptr, b.idx, b.nrows * (nw + 1), nw, seg);
+    k_win_bounds<<<nb(b.nrows * (nw + 1)), 256, 0, s>>>(b.ptr, b.idx, b.nrows * (nw + 1), nw, Sh::kCols, seg);
     GBK_LAUNCHED();
     k_win_tasks<<<(unsigned)std::min<int64_t>((ntasks + 7) / 8, (int64_t)num_sms() * 8), 256, 0, s>>>(
-        a.ptr, a.idx, seg, ntasks, nw, m, room, cls, d_hist);
+        a.ptr, a.idx, seg, ntasks, nw, Sh::kCols, m, room, cls, d_hist);
     GBK_LAUNCHED();
     k_win_order<<<nb(ntasks), 256, 0, s>>>(cls, 0, ntasks, d_hist, d_cursor, order);
     GBK_LAUNCHED();
@@ -544,9 +555,7 @@ int window_t(gbk_matrix* out, const CsrView& a, const CsrView& b, int64_t block_
     if (dev.get(&tcol, 4 * (size_t)max_room) || dev.get(&tval, sizeof(T) * (size_t)max_room) ||
         dev.get(&fin, 8 * (size_t)(ntasks + 1)))
         return GBK_SUCCESS;  // not done
-    const int smem = (int)(sizeof(T) + (flagged<SR>() ? 1 : 0)) * kWin * kWinWarps;
-    GBK_CUDA(cudaFuncSetAttribute(k_win_numeric<SR, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    const int per_sm = flagged<SR>() ? 2 : 3;
+    GBK_CUDA(cudaFuncSetAttribute(k_win_numeric<SR, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, Sh::kSmem));
     Owned own(s);
     if (own.get(0, 4 * (size_t)(n + 1))) return GBK_OUT_OF_MEMORY;
     std::vector<int32_t*> bcol(nblocks, nullptr);
@@ -565,9 +574,9 @@ int window_t(gbk_matrix* out, const CsrView& a, const CsrView& b, int64_t block_
         WindowArgs g{a.ptr, a.idx, a.val, b.idx, b.val, seg, nw, t0, order + t0, nheavy, run,
                      off, hroff[c], tcol, tval, count, d_next};
         if (run > 0) {
-            const int64_t ctas = std::min<int64_t>(std::max<int64_t>((run + kWinWarps - 1) / kWinWarps, g.nheavy),
-                                                   (int64_t)num_sms() * per_sm);
-            k_win_numeric<SR, T><<<(unsigned)ctas, 32 * kWinWarps, smem, s>>>(g);
+            const int64_t ctas = std::min<int64_t>(std::max<int64_t>((run + Sh::kWarps - 1) / Sh::kWarps, g.nheavy),
+                                                   (int64_t)num_sms() * Sh::kCtas);
+            k_win_numeric<SR, T><<<(unsigned)ctas, 32 * Sh::kWarps, Sh::kSmem, s>>>(g);
             GBK_LAUNCHED();
         }
         GBK_CUDA(cub::DeviceScan::ExclusiveSum(tmp, tb, count, fin, nt + 1, s));
@@ -634,9 +643,7 @@ int window_dispatch(gbk_matrix* out, const CsrView& a, const CsrView& b, int sr,
 int mxm_window(gbk_matrix* out, const CsrView& a, const CsrView& b, int vtype, int sr, int64_t block_entries, bool* done,
                cudaStream_t s) {
     *done = false;
-    if (a.nnz == 0 || b.nnz == 0 || b.ncols > (int64_t)kWin * kMaxWindows) return GBK_SUCCESS;
-    const int64_t nw = (b.ncols + kWin - 1) / kWin;
-    if (a.nrows * nw >= INT32_MAX) return GBK_SUCCESS;  // tasks are int32
+    if (a.nnz == 0 || b.nnz == 0 || b.ncols > kMaxColumns) return GBK_SUCCESS;
     return vtype == GBK_F32 ? window_dispatch<float>(out, a, b, sr, block_entries, done, s)
                             : window_dispatch<int32_t>(out, a, b, sr, block_entries, done, s);
 }

@@ -1,13 +1,13 @@
-"""gbk_mxm at the edges of its column windows (2,048 columns, at most 64 of them) and for the operands
-that the windows refuse (repeated or unsorted columns, too many columns, too few products a window),
-against sums in numpy: whole numbers, so every order of the sums gives the same value."""
+"""gbk_mxm at the edges of its column windows (1,280 columns for float sums, otherwise 2,048; 131,072 in all)
+and for the operands that the windows refuse (repeated or unsorted columns, too many columns, too few products
+a window), against sums in numpy: whole numbers, so every order of the sums gives the same value."""
 import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
 
-COLS = [1, 31, 2047, 2048, 2049, 4097, 64 * 2048 - 1, 64 * 2048, 64 * 2048 + 1]
+COLS = [1, 31, 1279, 1280, 1281, 2047, 2048, 2049, 4097, 64 * 2048 - 1, 64 * 2048, 64 * 2048 + 1]
 
 
 @pytest.fixture(scope="module")
@@ -155,11 +155,10 @@ def dense_rows(rng, rows, length, m):
 
 
 @pytest.mark.parametrize("blocks", [1, 5])
-@pytest.mark.parametrize("m,length", [(300, 4000), (2100, 700)])
+@pytest.mark.parametrize("m,length", [(300, 4000), (2100, 700), (1, 500), (1, 4000), (1, 16000), (8, 300), (1281, 200)])
 def test_float_sums(capi, monkeypatch, m, length, blocks):
     # Products rounded to 32 bits, their sums in 64: each product of non-negative terms and the final rounding
-    # add at most 2^-24 of the sum.  With 32-bit sums of thousands of terms: 8e-7 in blocks, before these had
-    # windows of 4,096 and more products worked on by whole CTAs.
+    # add at most 2^-24 of the sum.  32-bit sums of 500 terms in order: 3.0e-7, of 4,000: 7.9e-7.
     rows = 20
     rng = np.random.default_rng(m)
     (ap, ac, av), (bp, bc, bv) = dense_rows(rng, rows, length, m)
