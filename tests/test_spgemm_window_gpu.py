@@ -58,6 +58,30 @@ def product(ar, ac, av, br, bc, bv, m, sr):
     return keys[keep], out[keep]
 
 
+def room(ar, ac, br, bc, n, m, cols):
+    """Entries of room that the product asks for: per row and window of `cols` columns its products, at most the
+    window's columns."""
+    nw = (m + cols - 1) // cols
+    parts = np.zeros((max(int(ac.max()), int(br.max())) + 1, nw), np.int64)
+    np.add.at(parts, (br, bc // cols), 1)
+    tasks = np.zeros((n, nw), np.int64)
+    np.add.at(tasks, ar, parts[ac])
+    return np.minimum(tasks, np.minimum(cols, m - cols * np.arange(nw))).sum(axis=1)
+
+
+def set_blocks(monkeypatch, rows_room, blocks):
+    """Has a product with this room per row work in one block, in a block per row, or in a few of several rows
+    (a block has room for three entries per product allowed)."""
+    if blocks == "one":
+        monkeypatch.delenv("GBK_MXM_BLOCK_PRODUCTS", raising=False)
+        return
+    products = 1 if blocks == "rows" else max(1, int(rows_room.sum()) // 12)
+    monkeypatch.setenv("GBK_MXM_BLOCK_PRODUCTS", str(products))
+    if blocks == "few":
+        assert rows_room.sum() > 3 * products  # two blocks at least,
+        assert np.sort(rows_room)[:2].sum() <= 3 * products  # and some hold several rows
+
+
 def check(capi, A, B, want, m):
     C = A.mxm(B, semiring=want[0])
     rp, col, v = C.download_csr()
@@ -67,19 +91,17 @@ def check(capi, A, B, want, m):
     assert np.array_equal(v, want[2].astype(v.dtype))
 
 
-@pytest.mark.parametrize("block", [None, "1", "40009"])
+@pytest.mark.parametrize("blocks", ["one", "rows", "few"])
 @pytest.mark.parametrize("sr", ["plus_times", "plus_second", "plus_one", "min_plus", "min_second", "lor_land"])
 @pytest.mark.parametrize("m", COLS)
-def test_windows(capi, monkeypatch, m, sr, block):
-    if block:
-        monkeypatch.setenv("GBK_MXM_BLOCK_PRODUCTS", block)
-    else:
-        monkeypatch.delenv("GBK_MXM_BLOCK_PRODUCTS", raising=False)
+def test_windows(capi, monkeypatch, m, sr, blocks):
     rng = np.random.default_rng(m)
     n, k = 61, 47
     ar, ac = pattern(rng, n, k, 900)
     br, bc = pattern(rng, k, m, 6000)
     for dtype in (np.int32, np.float32):
+        cols = 1280 if dtype == np.float32 and sr.startswith("plus") else 2048
+        set_blocks(monkeypatch, room(ar, ac, br, bc, n, m, cols), blocks)
         av = rng.integers(-3, 4, len(ar)).astype(dtype)
         bv = rng.integers(-3, 4, len(br)).astype(dtype)
         if dtype == np.int32 and sr.startswith("min"):
@@ -92,9 +114,9 @@ def test_windows(capi, monkeypatch, m, sr, block):
 
 @pytest.mark.parametrize("sr", ["plus_times", "plus_second", "plus_one", "min_plus", "min_second", "lor_land"])
 @pytest.mark.parametrize("length", [511, 512, 513, 3000])
-def test_hub_rows(capi, monkeypatch, length, sr):
-    # a row that a CTA works on in several rounds, beside short ones
-    monkeypatch.delenv("GBK_MXM_BLOCK_PRODUCTS", raising=False)
+@pytest.mark.parametrize("blocks", ["one", "rows", "few"])
+def test_hub_rows(capi, monkeypatch, length, sr, blocks):
+    # a row whose windows a CTA works on, beside short ones
     rng = np.random.default_rng(length)
     n, k, m = 20, 3000, 2100
     ar, ac = pattern(rng, n, k, 300)
@@ -103,6 +125,8 @@ def test_hub_rows(capi, monkeypatch, length, sr):
     ar, ac = key // k, key % k
     br, bc = pattern(rng, k, m, 200_000)
     for dtype in (np.int32, np.float32):
+        cols = 1280 if dtype == np.float32 and sr.startswith("plus") else 2048
+        set_blocks(monkeypatch, room(ar, ac, br, bc, n, m, cols), blocks)
         av, bv = rng.integers(-3, 4, len(ar)).astype(dtype), rng.integers(-3, 4, len(br)).astype(dtype)
         A = capi.Matrix(*csr(ar, ac, n), av, ncols=k)
         B = capi.Matrix(*csr(br, bc, k), bv, ncols=m)
