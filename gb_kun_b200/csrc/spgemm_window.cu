@@ -451,14 +451,23 @@ struct Owned {
     }
 };
 
-// An (entry of A, window of 2,048 columns) pair costs about as much as a step of 32
-// products, and the tables of B's parts and of the tasks must not outgrow what the expansion
-// would hold (a hypersparse A or B has far more rows than products).
-bool window_pays(const CsrView& a, const CsrView& b, unsigned long long products) {
+// Windows or expansion, by their times in ns.  A (row, window) task costs 0.5,
+// mostly the scan of its columns, and an (entry of A, window) pair 0.2; integer
+// sums and or-and about 0.7 of that.  The expansion costs 0.085 a product and is
+// 0.15 ms slower to start, 0.85 ms where the sort takes several passes.  ms by
+// windows | by expansion, float sums, both close to the line: uniform graphs of
+// 2^15 vertices with 4, 16 and 32 entries a row 0.89 | 1.2, 2.0 | 1.75 and
+// 3.6 | 3.8, undirected R-MAT 2^16 with edge factors 1 and 2 2.0 | 1.9 and
+// 3.0 | 3.7.  Far from it: uniform 2^17, 16 a row, 24 | 5.2; R-MAT 2^16, edge
+// factor 4, 4.7 | 10.
+// The table of B's parts must not outgrow what the expansion would hold (a
+// hypersparse B has far more rows than products).  Windows counted as 2,048
+// columns each.
+bool window_pays(const CsrView& a, const CsrView& b, unsigned long long products, bool light) {
     const int64_t nw = (b.ncols + 2047) / 2048;
-    const unsigned long long most = 4 * products + 65536;
-    return (unsigned long long)a.nnz * nw <= most && (unsigned long long)a.nrows * nw <= most &&
-           (unsigned long long)b.nrows * (nw + 1) <= most;
+    const double windows = (light ? 0.7 : 1.0) * (0.5 * (double)a.nrows + 0.2 * (double)a.nnz) * (double)nw;
+    const double expansion = 0.085 * (double)products + (products > (1u << 18) ? 0.85e6 : 0.15e6);
+    return windows <= expansion && (unsigned long long)b.nrows * (nw + 1) <= 4 * products + 65536;
 }
 
 template <int SR, typename T>
@@ -481,7 +490,7 @@ int window_t(gbk_matrix* out, const CsrView& a, const CsrView& b, int64_t block_
     WindowHead head;
     GBK_CUDA(cudaMemcpyAsync(&head, d_head, sizeof(head), cudaMemcpyDeviceToHost, s));
     GBK_CUDA(cudaStreamSynchronize(s));
-    if (head.drops != head.row_drops || !window_pays(a, b, head.products)) return GBK_SUCCESS;
+    if (head.drops != head.row_drops || !window_pays(a, b, head.products, !Sh::kWide && !flagged<SR>())) return GBK_SUCCESS;
     // the parts of B's rows and the tasks' room
     int32_t *seg = nullptr, *order = nullptr;
     int64_t *room = nullptr, *off = nullptr;

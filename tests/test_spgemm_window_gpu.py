@@ -195,3 +195,28 @@ def test_float_sums(capi, monkeypatch, m, length, blocks):
     want = av.reshape(rows, length).astype(np.float64) @ bv.reshape(length, m).astype(np.float64)
     err = np.linalg.norm(v.reshape(rows, m) - want) / np.linalg.norm(want)
     assert err <= 2.0 ** -23
+
+
+@pytest.mark.parametrize("graph,scale,factor,windows", [
+    ("uniform", 16, 16, False), ("uniform", 15, 2, False), ("uniform", 15, 32, True), ("uniform", 14, 4, True),
+    ("rmat", 14, 8, True)])
+def test_route(capi, graph, scale, factor, windows):
+    # A product with far fewer products than (row, window) tasks is expanded, as it was before the windows (uniform
+    # 2^16, 16 entries a row: 2.6 ms, 6.8 by windows).  The same product with B's rows unsorted is always expanded:
+    # the number of launches tells the routes apart.
+    from gb_kun_b200 import graphgen as gg
+    g = getattr(gg, graph)(scale, factor, seed=3, undirected=graph == "rmat")
+    ptr, col = np.asarray(g.row_ptr).astype(np.int32), np.asarray(g.col).astype(np.int32)
+    val = np.random.default_rng(4).integers(1, 5, len(col)).astype(np.float32)  # whole sums: every order alike
+    rows = np.repeat(np.arange(g.n), np.diff(ptr))
+    o = np.lexsort((-col, rows))
+    A, U = capi.Matrix(ptr, col, val), capi.Matrix(ptr, col[o], val[o])
+    out, launches = [], []
+    for B in (A, U):
+        before = capi.launch_count()
+        C = A.mxm(B)
+        launches.append(capi.launch_count() - before)
+        out.append(C.download_csr())
+    for x, y in zip(*out):
+        assert np.array_equal(x, y)
+    assert (launches[0] != launches[1]) == windows
