@@ -7,6 +7,8 @@
 // column; here the CSC is produced by a radix sort on (col, row) keys, so
 // rows are ascending within each column and every run is deterministic.
 #include <algorithm>
+#include <mutex>
+#include <vector>
 
 #include <cub/cub.cuh>
 
@@ -160,10 +162,62 @@ int ensure_csc(gbk_matrix A, cudaStream_t s) {
     return GBK_SUCCESS;
 }
 
+// Arrays of the stream-ordered pool that a matrix owned.  Unlike cudaFree, which
+// waits for the device's work, cudaFreeAsync only orders the memory behind one
+// stream, so the wait comes first: that of the cudaFree of the matrix's tile
+// table, which is allowed while another thread captures a graph (a device
+// synchronise would end that capture, and so would the legacy stream).  If it is
+// refused, in a capture of this thread, the arrays wait for a later call.
+namespace {
+
+struct Released {
+    std::mutex lock;
+    cudaStream_t stream = nullptr;  // idle; created when the first pooled matrix is
+    std::vector<void*> waiting;
+};
+
+Released& released(int device) {
+    static Released r[64];
+    return r[device & 63];
+}
+
+cudaError_t release_stream(int device) {
+    Released& r = released(device);
+    std::lock_guard<std::mutex> g(r.lock);
+    return r.stream ? cudaSuccess : cudaStreamCreateWithFlags(&r.stream, cudaStreamNonBlocking);
+}
+
+void release_pooled(gbk_matrix A) {
+    Released& r = released(A->device);
+    CsrView& v = A->csr;
+    std::vector<void*> arrays;  // those that the wait covers
+    {
+        std::lock_guard<std::mutex> g(r.lock);
+        arrays.swap(r.waiting);
+    }
+    for (void* p : {(void*)v.ptr, (void*)v.idx, v.val}) arrays.push_back(p);
+    v.ptr = v.idx = nullptr;
+    v.val = nullptr;
+    cudaSetDevice(A->device);
+    if (cudaFree(v.tile_coord) == cudaSuccess) {
+        v.tile_coord = nullptr;
+        for (void* p : arrays) cudaFreeAsync(p, r.stream);
+    } else {
+        cudaGetLastError();
+        std::lock_guard<std::mutex> g(r.lock);
+        r.waiting.insert(r.waiting.end(), arrays.begin(), arrays.end());
+    }
+}
+
+}  // namespace
+
 int adopt_csr(gbk_matrix* out, int64_t nrows, int64_t ncols, int64_t nnz, int32_t* ptr, int32_t* idx, void* val,
               gbk_dtype vtype, cudaStream_t s) {
+    int device = 0;
+    GBK_CUDA(cudaGetDevice(&device));
+    GBK_CUDA(release_stream(device));
     gbk_matrix A = new gbk_matrix_s();
-    cudaGetDevice(&A->device);
+    A->device = device;
     A->vtype = vtype;
     A->pooled = true;
     CsrView& v = A->csr;
@@ -243,14 +297,7 @@ int gbk_matrix_destroy(gbk_matrix A) {
     free_formats(A);
     int current = 0;
     cudaGetDevice(&current);
-    if (A->pooled) {
-        // unlike cudaMalloc'd arrays, the pool's are freed without waiting for work in flight
-        cudaSetDevice(A->device);
-        cudaDeviceSynchronize();
-        for (void* p : {(void*)A->csr.ptr, (void*)A->csr.idx, A->csr.val}) cudaFreeAsync(p, 0);
-        A->csr.ptr = A->csr.idx = nullptr;
-        A->csr.val = nullptr;
-    }
+    if (A->pooled) release_pooled(A);
     free_view(A->csr);
     free_view(A->csc);
     cudaFree(A->xcopy);
