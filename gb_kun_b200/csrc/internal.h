@@ -67,7 +67,7 @@ struct gbk_matrix_s {
     gbk::CsrView csr;           // A
     gbk::CsrView csc;           // A^T (built lazily)
     bool has_csc = false;
-    bool pooled = false;  // csr.ptr, idx and val come from the stream-ordered pool
+    bool pooled = false;  // csr.ptr, idx and val come from the products' pool (result_alloc)
     int8_t pattern_symmetric = -1;  // -1 unknown; gbk_matrix_pattern_symmetric
     int32_t* coldeg = nullptr;      // entries per column, built by the first gbk_pagerank
     int64_t coldeg_zero = 0;        // columns without entries (valid with coldeg)
@@ -107,8 +107,12 @@ int ensure_csc(gbk_matrix A, cudaStream_t s);
 void free_single_cache(gbk_matrix A);
 void free_batches(gbk_matrix A);  // batched.cu
 int build_tiles(CsrView& v, int elem_bytes, cudaStream_t s);
-// A matrix around arrays of the stream-ordered pool, which it owns from then on; on an error
-// they stay the caller's.  Synchronises the stream.  matrix.cu
+// Memory for a product's arrays, from the stream-ordered pool that products share (current
+// device); release_results gives back what dropped products left in it.  matrix.cu
+int result_alloc(void** p, size_t bytes, cudaStream_t s);
+void release_results();
+// A matrix around such arrays, which it owns from then on; on an error they stay the caller's.
+// Synchronises the stream.
 int adopt_csr(gbk_matrix* out, int64_t nrows, int64_t ncols, int64_t nnz, int32_t* ptr, int32_t* idx, void* val,
               gbk_dtype vtype, cudaStream_t s);
 // Unmasked product in column windows (spgemm_window.cu); *done = false when

@@ -296,6 +296,7 @@ int gbk_server_create(gbk_matrix A, const gbk_server_config* cfg, gbk_server* ou
         S->budget = c.memory_budget;
     } else {
         size_t fr = 0, tot = 0;
+        release_results();  // what dropped products left is free memory too
         cudaMemGetInfo(&fr, &tot);
         S->budget = (int64_t)(0.8 * (double)fr);
     }

@@ -431,8 +431,7 @@ __global__ void k_win_row_room(const int64_t* __restrict__ off, int64_t nrows, i
 
 unsigned nb(int64_t n) { return (unsigned)std::max<int64_t>(1, (n + 255) / 256); }
 
-// ptr, col and val of C from the stream-ordered pool, freed unless handed over
-// (cudaMalloc and cudaFree of a result of 46 M entries took 2 ms a call).
+// ptr, col and val of C, freed unless handed over.
 struct Owned {
     cudaStream_t s;
     void* p[3] = {nullptr, nullptr, nullptr};
@@ -443,11 +442,13 @@ struct Owned {
             if (q) cudaFreeAsync(q, s);
     }
     int get(int k, size_t bytes) {
-        if (cudaMallocAsync(&p[k], bytes, s) == cudaSuccess) return GBK_SUCCESS;
-        cudaGetLastError();
-        p[k] = nullptr;
-        set_error("gbk_mxm: out of device memory for the result");
-        return GBK_OUT_OF_MEMORY;
+        const int rc = result_alloc(&p[k], bytes, s);
+        if (rc == GBK_OUT_OF_MEMORY) set_error("gbk_mxm: out of device memory for the result");
+        return rc;
+    }
+    int get_entries(size_t entries, size_t elem) {
+        const int rc = get(1, 4 * entries);
+        return rc ? rc : get(2, elem * entries);
     }
 };
 
@@ -566,7 +567,7 @@ int window_t(gbk_matrix* out, const CsrView& a, const CsrView& b, int64_t block_
         return GBK_SUCCESS;  // not done
     GBK_CUDA(cudaFuncSetAttribute(k_win_numeric<SR, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, Sh::kSmem));
     Owned own(s);
-    if (own.get(0, 4 * (size_t)(n + 1))) return GBK_OUT_OF_MEMORY;
+    if (const int rc = own.get(0, 4 * (size_t)(n + 1))) return rc;
     std::vector<int32_t*> bcol(nblocks, nullptr);
     std::vector<T*> bval(nblocks, nullptr);
     std::vector<int64_t> bcnt(nblocks, 0);
@@ -596,7 +597,7 @@ int window_t(gbk_matrix* out, const CsrView& a, const CsrView& b, int64_t block_
                     (long long)(total + bcnt[c]));
         const size_t entries = (size_t)std::max<int64_t>(bcnt[c], 1);
         if (nblocks == 1) {
-            if (own.get(1, 4 * entries) || own.get(2, sizeof(T) * entries)) return GBK_OUT_OF_MEMORY;
+            if (const int rc = own.get_entries(entries, sizeof(T))) return rc;
             bcol[c] = (int32_t*)own.p[1];
             bval[c] = (T*)own.p[2];
         } else if (dev.get(&bcol[c], 4 * entries) || dev.get(&bval[c], sizeof(T) * entries)) {
@@ -615,7 +616,7 @@ int window_t(gbk_matrix* out, const CsrView& a, const CsrView& b, int64_t block_
     }
     if (nblocks > 1) {
         const size_t entries = (size_t)std::max<int64_t>(total, 1);
-        if (own.get(1, 4 * entries) || own.get(2, sizeof(T) * entries)) return GBK_OUT_OF_MEMORY;
+        if (const int rc = own.get_entries(entries, sizeof(T))) return rc;
         int64_t at = 0;
         for (size_t c = 0; c < nblocks; ++c) {
             if (bcnt[c] > 0) {

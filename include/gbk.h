@@ -93,6 +93,9 @@ int64_t gbk_launch_count(void);
  * device on first use. */
 int gbk_matrix_create_csr(gbk_matrix* out, int64_t nrows, int64_t ncols, int64_t nnz, const int32_t* row_ptr,
                           const int32_t* col, const void* val, gbk_dtype vtype, int on_device, void* stream);
+/* Waits for the device's work, then frees.  Up to 1 GiB of what dropped
+ * gbk_mxm results held stays reserved for the next ones (gbk_server_create
+ * gives it back before it counts the free memory). */
 int gbk_matrix_destroy(gbk_matrix A);
 int gbk_matrix_get_info(gbk_matrix A, gbk_matrix_info* info);
 /* Device pointers of the CSR (transpose = 0) or CSC (transpose = 1) arrays. */

@@ -1,5 +1,6 @@
 """Products whose arrays come from the stream-ordered pool: dropping one waits for work that still reads it, on any
 stream, and disturbs neither a capture nor a first call in another thread."""
+import ctypes
 import threading
 
 import numpy as np
@@ -112,3 +113,38 @@ def test_destroy_beside_first_calls(capi, graph, oracle):
         stop.set()
         t.join()
     assert not errors, errors
+
+
+def default_pool():
+    rt = ctypes.CDLL("libcudart.so.12")
+    pool = ctypes.c_void_p()
+    assert rt.cudaDeviceGetDefaultMemPool(ctypes.byref(pool), 0) == 0
+    return rt, pool
+
+
+def test_what_dropped_products_leave(capi):
+    """The device's default pool, which others share, keeps what it had; a server counts what products left as free."""
+    from gb_kun_b200.serve import Server
+    rt, pool = default_pool()
+    reserved = ctypes.c_uint64()
+
+    def now():
+        torch.cuda.synchronize()
+        assert rt.cudaMemPoolGetAttribute(pool, 5, ctypes.byref(reserved)) == 0  # cudaMemPoolAttrReservedMemCurrent
+        return reserved.value
+
+    p = ctypes.c_void_p()  # another user of the default pool, with 5 GiB that it will want again
+    assert rt.cudaMallocAsync(ctypes.byref(p), ctypes.c_size_t(5 << 30), None) == 0
+    assert rt.cudaFreeAsync(p, None) == 0
+    g = gg.rmat(14, 16, seed=9, undirected=True)
+    A = capi.Matrix.from_graph(g)
+    A.mxm(A).close()
+    before = now()
+    assert before >= 5 << 30
+    C = A.mxm(A)  # 40 M entries
+    with_c = Server(A).memory()[1]
+    size = 8 * C.nnz
+    C.close()
+    assert now() == before
+    assert Server(A).memory()[1] >= with_c + 0.75 * size  # a server's budget is 80 % of the free memory
+    assert rt.cudaMemPoolTrimTo(pool, ctypes.c_size_t(0)) == 0
