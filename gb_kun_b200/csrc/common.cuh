@@ -9,6 +9,7 @@
 #include <type_traits>
 
 #include "gbk_types.h"
+#include "ranges.h"
 
 namespace gbk {
 

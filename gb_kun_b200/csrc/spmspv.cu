@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(kPushThreads) k_push(PushArgs a) {
         }
         bool heavy = deg >= kHeavyRow;
         if (heavy) {
-            const int32_t np = (deg + kPiece - 1) / kPiece;
+            const int32_t np = pieces_of(deg, kPiece);
             const int32_t at = atomicAdd(a.npieces, np);
             if (at >= 0 && at <= a.room - np)
                 for (int32_t i = 0; i < np; ++i) a.pieces[at + i] = make_int2((int32_t)k, beg + i * kPiece);
@@ -173,7 +173,8 @@ __global__ void __launch_bounds__(kPushThreads) k_push(PushArgs a) {
             lone &= lone - 1;
             const int32_t eb = __shfl_sync(kFull, beg, j), d = __shfl_sync(kFull, deg, j);
             const T xj = __shfl_sync(kFull, x, j);
-            for (int32_t t0 = 0; t0 < d; t0 += 32) push_edge<SR, T>(a, t0 + lane < d, (int64_t)eb + t0 + lane, xj, lane);
+            for (uint32_t t0 = 0; t0 < (uint32_t)d; t0 += 32)
+                push_edge<SR, T>(a, t0 + lane < (uint32_t)d, (int64_t)eb + t0 + lane, xj, lane);
         }
     }
 }
@@ -190,9 +191,9 @@ __global__ void __launch_bounds__(kPushThreads) k_push_pieces(PushArgs a) {
         if (pc.x < 0) continue;
         T x = T(0);
         if constexpr (push_kind<SR>() != kPushOne) x = __ldg((const T*)a.xv + pc.x);
-        const int32_t end = min(pc.y + kPiece, __ldg(a.ptr + __ldg(a.ids + pc.x) + 1));
+        const uint32_t end = piece_end(pc.y, kPiece, __ldg(a.ptr + __ldg(a.ids + pc.x) + 1));
 #pragma unroll 4
-        for (int32_t e0 = pc.y; e0 < end; e0 += 32) push_edge<SR, T>(a, e0 + lane < end, (int64_t)e0 + lane, x, lane);
+        for (uint32_t e0 = pc.y; e0 < end; e0 += 32) push_edge<SR, T>(a, e0 + lane < end, (int64_t)e0 + lane, x, lane);
     }
 }
 
