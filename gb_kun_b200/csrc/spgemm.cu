@@ -708,11 +708,12 @@ __global__ void __launch_bounds__(256, 8) k_tc_warp(TcArgs a) {
     for (int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < ni; i += nw) {
         const int2 it = a.items[i];
         const int32_t b = a.op[it.x], d = a.op[it.x + 1] - b;
-        const int32_t end = it.y + min(a.ap[it.x + 1] - it.y, a.run);
+        const int32_t* __restrict__ row = a.ai + it.y;
+        const int32_t len = min(a.ap[it.x + 1] - it.y, a.run);
         set.build(a.oi + b, d, lane, 32);
         __syncwarp();
-        for (int32_t e = it.y; e < end; e += 32)
-            mine += tc_lookup(set, a.op, a.oi, it.x, d, e + lane < end ? a.ai[e + lane] : -1, lane, slots);
+        for (int32_t e = 0; e < len; e += 32)
+            mine += tc_lookup(set, a.op, a.oi, it.x, d, e + lane < len ? row[e + lane] : -1, lane, slots);
         __syncwarp();
     }
     tc_add_total<256>(mine, a.total);
@@ -747,7 +748,8 @@ __global__ void __launch_bounds__(THREADS, 2048 / THREADS) k_tc_cta(TcArgs a) {
         if (i >= ni) break;
         const int2 it = a.items[i];
         const int32_t b = a.op[it.x], d = a.op[it.x + 1] - b;
-        const int32_t end = it.y + min(a.ap[it.x + 1] - it.y, a.run);
+        const int32_t* __restrict__ row = a.ai + it.y;
+        const int32_t len = min(a.ap[it.x + 1] - it.y, a.run);
         if (threadIdx.x == 0) {
             s_item[turn ^ 1] = atomicAdd(a.next, 1);
             s_group = 0;
@@ -757,9 +759,9 @@ __global__ void __launch_bounds__(THREADS, 2048 / THREADS) k_tc_cta(TcArgs a) {
         for (;;) {
             int32_t g = 0;
             if (lane == 0) g = atomicAdd(&s_group, 1);
-            const int32_t e = it.y + 32 * __shfl_sync(0xffffffffu, g, 0);
-            if (e >= end) break;
-            mine += tc_lookup(set, a.op, a.oi, it.x, d, e + lane < end ? a.ai[e + lane] : -1, lane, slots);
+            const int32_t e = 32 * __shfl_sync(0xffffffffu, g, 0);
+            if (e >= len) break;
+            mine += tc_lookup(set, a.op, a.oi, it.x, d, e + lane < len ? row[e + lane] : -1, lane, slots);
         }
         __syncthreads();
         set.clear(a.oi + b, d, threadIdx.x, THREADS);
