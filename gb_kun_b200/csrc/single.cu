@@ -267,7 +267,7 @@ __device__ void expand_light(const int32_t* __restrict__ qc, int32_t fc, const i
         const int32_t u = k < fc ? qc[k] : -1;
         const int32_t beg = u >= 0 ? rp[u] : 0, deg = u >= 0 ? rp[u + 1] - beg : 0;
         const bool heavy = deg >= kHeavy;
-        const int32_t nch = heavy ? (deg + kChunk - 1) / kChunk : 0;
+        const int32_t nch = heavy ? pieces_of(deg, kChunk) : 0;
         const int32_t ich = warp_incl_scan(nch);
         const int32_t tch = __shfl_sync(kAll, ich, 31);
         if (tch) {
@@ -313,16 +313,17 @@ __device__ void expand_heavy(const Chunk* __restrict__ chunks, int32_t nch, cons
     const int64_t gw = ((int64_t)blockIdx.x * kT + threadIdx.x) >> 5, nw = ((int64_t)gridDim.x * kT) >> 5;
     for (int64_t c = gw; c < nch; c += nw) {
         const Chunk ch = chunks[c];
-        const int32_t end = min(ch.beg + kChunk, rp[ch.u + 1]);
+        const int32_t len = piece_end(ch.beg, kChunk, rp[ch.u + 1]) - ch.beg;
         const typename Op::V val = op.load(ch.u);
-        for (int32_t e0 = ch.beg; e0 < end; e0 += 32 * kBatch) {
+        for (int32_t e0 = 0; e0 < len; e0 += 32 * kBatch) {
             bool valid[kBatch];
             typename Op::V vals[kBatch];
             int32_t e[kBatch];
 #pragma unroll
             for (int k = 0; k < kBatch; ++k) {
-                e[k] = e0 + 32 * k + lane;
-                valid[k] = e[k] < end;
+                const int32_t at = e0 + 32 * k + lane;
+                valid[k] = at < len;
+                e[k] = valid[k] ? ch.beg + at : 0;
                 vals[k] = val;
             }
             op.template edges<kBatch>(valid, vals, e);
@@ -438,10 +439,10 @@ __global__ void __launch_bounds__(kT) k_bfs1_light(Bfs1Bufs b, Bfs1State* st) {
             const int32_t beg = un ? b.crp[v] : 0, deg = un ? b.crp[v + 1] - beg : 0;
             bool found = false;
             if (deg < kHeavy)
-                for (int32_t e = beg; e < beg + deg && !found; e += kBatch) {
+                for (int32_t o = 0; o < deg && !found; o += kBatch) {
                     int32_t u[kBatch];  // neighbouring entries: mostly one sector
 #pragma unroll
-                    for (int k = 0; k < kBatch; ++k) u[k] = e + k < beg + deg ? __ldg(b.crow + e + k) : -1;
+                    for (int k = 0; k < kBatch; ++k) u[k] = o + k < deg ? __ldg(b.crow + beg + o + k) : -1;
 #pragma unroll
                     for (int k = 0; k < kBatch; ++k) found |= u[k] >= 0 && ((bc[u[k] >> 5] >> (u[k] & 31)) & 1u);
                 }
@@ -451,9 +452,9 @@ __global__ void __launch_bounds__(kT) k_bfs1_light(Bfs1Bufs b, Bfs1State* st) {
                 hubs &= hubs - 1;
                 const int32_t hb = __shfl_sync(kAll, beg, h), hd = __shfl_sync(kAll, deg, h);
                 bool hf = false;
-                for (int32_t e0 = 0; e0 < hd && !hf; e0 += 32) {
+                for (uint32_t e0 = 0; e0 < (uint32_t)hd && !hf; e0 += 32) {
                     bool f = false;
-                    if (e0 + lane < hd) {
+                    if (e0 + lane < (uint32_t)hd) {
                         const int32_t u = b.crow[hb + e0 + lane];
                         f = (bc[u >> 5] >> (u & 31)) & 1u;
                     }
