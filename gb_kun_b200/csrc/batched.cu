@@ -1379,14 +1379,14 @@ __global__ void __launch_bounds__(kBT) k_sssp_push(const ColCfg* __restrict__ cf
     const int64_t nw = ((int64_t)gridDim.x * kBT) >> 5;
     for (int64_t it0 = gw; it0 < nitems; it0 += 32 * nw) {
         const int64_t it = it0 + lane * nw;
-        int32_t my_row = 0, my_beg = 0, my_end = 0;
+        int32_t my_row = 0, my_beg = 0, my_len = 0;
         uint32_t my_cm = 0;
         if (it < nitems) {
             my_row = cfg->item_row[it];
             my_cm = chg_in[my_row] & act;
             if (my_cm) {
                 my_beg = cfg->item_beg[it];
-                my_end = min(my_beg + C, rp[my_row + 1]);
+                my_len = piece_end(my_beg, C, rp[my_row + 1]) - my_beg;
             }
         }
         unsigned todo = __ballot_sync(kFull, my_cm != 0);
@@ -1394,15 +1394,15 @@ __global__ void __launch_bounds__(kBT) k_sssp_push(const ColCfg* __restrict__ cf
             const int src = __ffs(todo) - 1;
             todo &= todo - 1;
             const int32_t row = __shfl_sync(kFull, my_row, src);
-            const int32_t beg = __shfl_sync(kFull, my_beg, src), end = __shfl_sync(kFull, my_end, src);
+            const int32_t beg = __shfl_sync(kFull, my_beg, src), len = __shfl_sync(kFull, my_len, src);
             const bool mine = (__shfl_sync(kFull, my_cm, src) >> lane) & 1;
             const int32_t dv = mine ? __ldcg(dist + (int64_t)row * 32 + lane) : INT_MAX;
-            for (int32_t e0 = beg; e0 < end; e0 += 32) {
-                const int cnt = min(32, end - e0);
+            for (int32_t e0 = 0; e0 < len; e0 += 32) {
+                const int cnt = min(32, len - e0);
                 int32_t cl = 0, wl = 0;
                 if (lane < cnt) {
-                    cl = __ldcs(col + e0 + lane);
-                    wl = weight_at(cfg, e0 + lane);
+                    cl = __ldcs(col + beg + e0 + lane);
+                    wl = weight_at(cfg, beg + e0 + lane);
                 }
                 for (int j = 0; j < cnt; j += kRelax) {
                     int32_t cand[kRelax], have[kRelax];
