@@ -156,8 +156,8 @@ __global__ void __launch_bounds__(256) k_win_tasks(const int32_t* __restrict__ a
     for (int64_t t = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < ntasks; t += nwarps) {
         const int32_t row = (int32_t)t / nw, w = (int32_t)t - row * nw;  // tasks are int32
         long long sum = 0;
-        const int32_t a1 = aptr[row + 1];
-        for (int32_t e = aptr[row] + lane; e < a1; e += 32) {
+        const uint32_t a1 = aptr[row + 1];
+        for (uint32_t e = aptr[row] + lane; e < a1; e += 32) {
             const int32_t* s = seg + (int64_t)aidx[e] * (nw + 1) + w;
             sum += s[1] - s[0];
         }
@@ -231,7 +231,7 @@ struct WindowArgs {
 
 // A warp's sums of one window over the entries [a0, a1) of a row of A.
 template <int SR, typename T>
-__device__ __forceinline__ void window_sums(const WindowArgs& g, int w, int32_t a0, int32_t a1,
+__device__ __forceinline__ void window_sums(const WindowArgs& g, int w, uint32_t a0, uint32_t a1,
                                             typename Shape<SR, T>::Sum* acc, uint8_t* seen, int lane) {
     using S = Semiring<SR, T>;
     using Sum = typename Shape<SR, T>::Sum;
@@ -242,7 +242,7 @@ __device__ __forceinline__ void window_sums(const WindowArgs& g, int w, int32_t 
     const int32_t col0 = w * Shape<SR, T>::kCols;
     const int32_t* __restrict__ seg = g.seg + w;
     for (; a0 < a1; a0 += 32) {
-        int32_t sb = 0, se = 0;
+        uint32_t sb = 0, se = 0;
         T av = T(0);
         if (a0 + lane < a1) {
             const int32_t k = g.aidx[a0 + lane];
@@ -251,7 +251,7 @@ __device__ __forceinline__ void window_sums(const WindowArgs& g, int w, int32_t 
             se = __ldg(seg + (int64_t)k * (g.nw + 1) + 1);
         }
         unsigned todo = __ballot_sync(kAll, se > sb);
-        int32_t p = 0, e = 0;  // what is left of the current part of a row of B
+        uint32_t p = 0, e = 0;  // what is left of the current part of a row of B
         T a = T(0);
         while (todo || p < e) {
             int32_t c[kSteps];
@@ -360,9 +360,9 @@ __global__ void __launch_bounds__(32 * Shape<SR, T>::kWarps, Shape<SR, T>::kCtas
             const int32_t task = g.order[s_next];
             const int32_t row = task / g.nw, w = task - row * g.nw;
             const int32_t a0 = g.aptr[row], a1 = g.aptr[row + 1];
-            const int32_t per = min(32, (a1 - a0 + kWarps - 1) / kWarps);  // entries of A per warp and turn
+            const int32_t per = min(32, pieces_of(a1 - a0, kWarps));  // entries of A per warp and turn
             for (int64_t from = (int64_t)a0 + warp * per; from < a1; from += kWarps * per)
-                window_sums<SR, T>(g, w, (int32_t)from, (int32_t)(from + per < a1 ? from + per : a1), acc, seen, lane);
+                window_sums<SR, T>(g, w, (uint32_t)from, (uint32_t)(from + per < a1 ? from + per : a1), acc, seen, lane);
             __syncthreads();
             for (int q = threadIdx.x; q < kCols; q += 32 * kWarps) {
                 Sum tot = S::identity();
