@@ -36,6 +36,7 @@ constexpr int kBinWarps = kBinThreads / 32;
 #define GBK_SPLIT_NNZ 2048
 #endif
 constexpr int kSplitNnz = GBK_SPLIT_NNZ;
+static_assert(kSplitNnz <= kLookAhead, "ends of chunks are formed past the last entry");
 constexpr int kLaneNnz = 2;  // entries per lane of a group
 // bins: 0 empty, 1..6 -> G = 1,2,4,8,16,32, 7 warp, 8 split
 constexpr int kNumBins = 9;

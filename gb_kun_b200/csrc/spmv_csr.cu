@@ -274,7 +274,8 @@ int spmv_csr(const CsrView& v, int sr, int accum, int dtype, const void* x, void
         }
         return spmv_chunks(v.chunks, v, sr, accum, dtype, x, y, mask, mask_dtype, mask_mode, s);
     }
-    if (v.kernel != kKernelMerge && assoc_semiring(sr) && v.nrows > 0) {
+    // (a matrix of nearly 2^31 entries takes the merge kernel: the bins look ahead past its end)
+    if (v.kernel != kKernelMerge && assoc_semiring(sr) && v.nrows > 0 && can_look_ahead(v.nnz)) {
         if (!v.bins) {
             int rc = build_bins(v, (int)dtype_size(dtype), &v.bins, s);
             if (rc) return rc;
