@@ -120,8 +120,10 @@ int adopt_csr(gbk_matrix* out, int64_t nrows, int64_t ncols, int64_t nnz, int32_
 int mxm_window(gbk_matrix* out, const CsrView& a, const CsrView& b, int vtype, int sr, int64_t block_entries,
                bool* done, cudaStream_t s);
 
+void set_error(const char* fmt, ...);  // core.cu
+
 // Device scratch from the stream-ordered pool (reused across calls), freed
-// on the stream on every exit.
+// on the stream on every exit.  A refused request leaves an error message.
 struct StreamScratch {
     cudaStream_t s;
     std::vector<void*> p;
@@ -135,6 +137,7 @@ struct StreamScratch {
         void* q = nullptr;
         if (cudaMallocAsync(&q, bytes < 16 ? 16 : bytes, s) != cudaSuccess) {
             cudaGetLastError();
+            set_error("out of device memory (%zu bytes of scratch)", bytes);
             return GBK_OUT_OF_MEMORY;
         }
         p.push_back(q);

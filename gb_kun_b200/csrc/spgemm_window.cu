@@ -480,7 +480,7 @@ int window_t(gbk_matrix* out, const CsrView& a, const CsrView& b, int64_t block_
     if (ntasks >= INT32_MAX) return GBK_SUCCESS;  // tasks are int32
     StreamScratch dev(s);
     WindowHead* d_head = nullptr;
-    if (dev.get(&d_head, 512)) return GBK_OUT_OF_MEMORY;
+    if (dev.get(&d_head, 512)) return GBK_SUCCESS;  // not done, as for all scratch: the expansion may still fit
     unsigned long long* d_next = (unsigned long long*)d_head + 4;
     int32_t* d_hist = (int32_t*)(d_next + 2);
     int32_t* d_cursor = d_hist + kClasses;
@@ -499,7 +499,7 @@ int window_t(gbk_matrix* out, const CsrView& a, const CsrView& b, int64_t block_
     if (dev.get(&seg, 4 * (size_t)b.nrows * (nw + 1)) || dev.get(&order, 4 * (size_t)ntasks) ||
         dev.get(&room, 8 * (size_t)(ntasks + 1)) || dev.get(&off, 8 * (size_t)(ntasks + 1)) ||
         dev.get(&cls, (size_t)ntasks))
-        return GBK_SUCCESS;  // not done: the expansion may still fit
+        return GBK_SUCCESS;
     k_win_bounds<<<nb(b.nrows * (nw + 1)), 256, 0, s>>>(b.ptr, b.idx, b.nrows * (nw + 1), nw, Sh::kCols, seg);
     GBK_LAUNCHED();
     k_win_tasks<<<(unsigned)std::min<int64_t>((ntasks + 7) / 8, (int64_t)num_sms() * 8), 256, 0, s>>>(
@@ -510,7 +510,7 @@ int window_t(gbk_matrix* out, const CsrView& a, const CsrView& b, int64_t block_
     size_t tb = 0;
     cub::DeviceScan::ExclusiveSum(nullptr, tb, room, off, ntasks + 1, s);
     void* tmp = nullptr;
-    if (dev.get(&tmp, tb)) return GBK_OUT_OF_MEMORY;
+    if (dev.get(&tmp, tb)) return GBK_SUCCESS;
     GBK_CUDA(cub::DeviceScan::ExclusiveSum(tmp, tb, room, off, ntasks + 1, s));
     count_launch(1);
     int64_t total_room = 0;
@@ -522,7 +522,7 @@ int window_t(gbk_matrix* out, const CsrView& a, const CsrView& b, int64_t block_
     std::vector<int64_t> cuts{0, n}, hroff{0, total_room};  // cut rows and the room before them
     if (total_room > block_entries) {
         int64_t* roff = nullptr;
-        if (dev.get(&roff, 8 * (size_t)(n + 1))) return GBK_OUT_OF_MEMORY;
+        if (dev.get(&roff, 8 * (size_t)(n + 1))) return GBK_SUCCESS;
         k_win_row_room<<<nb(n + 1), 256, 0, s>>>(off, n, nw, roff);
         GBK_LAUNCHED();
         std::vector<int64_t> all(n + 1);
@@ -542,7 +542,7 @@ int window_t(gbk_matrix* out, const CsrView& a, const CsrView& b, int64_t block_
     if (nblocks > 1) {  // each block's tasks in an order of their own
         int32_t* d_bhist = nullptr;  // per block: tasks per class, then cursors
         const size_t bytes = 4 * 2 * kClasses * nblocks;
-        if (dev.get(&d_bhist, bytes)) return GBK_SUCCESS;  // not done
+        if (dev.get(&d_bhist, bytes)) return GBK_SUCCESS;
         GBK_CUDA(cudaMemsetAsync(d_bhist, 0, bytes, s));
         for (size_t c = 0; c < nblocks; ++c) {
             const int64_t t0 = cuts[c] * nw, nt = (cuts[c + 1] - cuts[c]) * nw;
@@ -564,7 +564,7 @@ int window_t(gbk_matrix* out, const CsrView& a, const CsrView& b, int64_t block_
     int64_t* fin = nullptr;
     if (dev.get(&tcol, 4 * (size_t)max_room) || dev.get(&tval, sizeof(T) * (size_t)max_room) ||
         dev.get(&fin, 8 * (size_t)(ntasks + 1)))
-        return GBK_SUCCESS;  // not done
+        return GBK_SUCCESS;
     GBK_CUDA(cudaFuncSetAttribute(k_win_numeric<SR, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, Sh::kSmem));
     Owned own(s);
     if (const int rc = own.get(0, 4 * (size_t)(n + 1))) return rc;
