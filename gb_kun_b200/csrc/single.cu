@@ -250,9 +250,10 @@ __device__ __forceinline__ void queue_append(const bool (&found)[U], const int32
 // lane), longer rows appended to `chunks` for expand_heavy.  Op::load(u)
 // gives the per-row value passed to op.edges.  Bound by the chain entry ->
 // neighbour's state -> atomic -> queue, so an operator gets kBatch entries a
-// lane at a time and overlaps their chains (four against one:
-// SSSP on R-MAT 2^20 2.32 -> 1.90 ms, on 300,001 uniform vertices 2.21 -> 1.82;
-// BFS on 700,001 uniform vertices 371 -> 298 us, R-MAT 2^21 353 -> 319).
+// lane at a time and overlaps their chains (four against one, both sides in turn:
+// SSSP on R-MAT 2^20 2.39 -> 1.95 ms, on 300,001 uniform vertices 2.10 -> 1.67;
+// BFS on 700,001 uniform vertices 379 -> 290 us, on R-MAT 2^21 344 to 415 us by
+// source, 1.04 to 1.19 times as fast).
 constexpr int kBatch = 4;
 
 template <class Op>

@@ -20,7 +20,8 @@
 // A A of an undirected R-MAT graph of 2^14 vertices, 157 M products, 46 M
 // entries: 1.3 ms a call, where it took 11.7 ms by expansion and sorting, which
 // move every product through memory several times; what is left is the sums
-// (0.84 ms) and the result's move to its place (0.26 ms).
+// (0.82 ms) and the result's move to its place (0.24 ms).  2^15, 445 M products,
+// in two blocks: 4.5 ms, 29 by expansion.
 #include <cub/cub.cuh>
 
 #include <algorithm>
